@@ -1,0 +1,61 @@
+"""The key encoder for 256-token blocks, bit for bit against the CPU oracle at the places where it
+can go wrong: every outlier count it takes (and one it leaves to the general encoder), tokens split
+between the hot ring and the caller's tensor, equal magnitudes, channels whose levels round together
+(constants, a large zero-point over a small range), every grid and element type."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+H, W, S = 2, 512, 256
+
+
+def _tokens(rng, n, dt):
+    """(n, H, 128) float32 holding values of `dt`, with the awkward channels named above."""
+    import torch
+
+    x = rng.standard_normal((n, H, 128)).astype(np.float32) * np.exp(rng.normal(0, 1, (1, H, 128)))
+    x[:, :, 3] *= 20.0
+    x[:, 0, 8] = 0.0                                              # all zero
+    x[:, 0, 9] = 1.25                                             # constant
+    x[:, 0, 10] = 300.0 + 0.25 * rng.integers(0, 2, n)            # two values far from zero
+    x[:, 0, 11] = rng.integers(-3, 4, n)                          # many equal magnitudes
+    x[:, 0, 12] = 1.0e-6 * rng.standard_normal(n)
+    x[:, 1, 13] = np.linspace(-1.0, 1.0, n)                       # all large ones side by side
+    x[:, 1, 14] = 40.0 + rng.standard_normal(n)
+    x[::7, 1, 15] = -0.0
+    x[5:9, 1, :] = 9.0                                            # more outliers than fixed slots
+    return torch.from_numpy(x.astype(np.float32)).to(getattr(torch, dt))
+
+
+@pytest.mark.parametrize("dt", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("mode", ["nf4_asym", "nf4", "uniform"])
+@pytest.mark.parametrize("frac,k", [(0.0, 0), (0.003, 1), (0.02, 5), (0.032, 8), (0.036, 9)])
+def test_key_blocks_equal_the_oracle(dt, mode, frac, k):
+    import torch
+
+    from oracle import tq_oracle as orc
+    from turboquant_pro_b200 import KVContext
+
+    assert orc.outlier_count(S, frac) == k or frac == 0.0
+    n = 1100
+    t = _tokens(np.random.default_rng(11), n, dt)
+    ctx = KVContext(n_layers=1, n_seqs=1, n_kv_heads=H, n_q_heads=H, value_bits=3, hot_window=W,
+                    max_tokens_per_seq=n, kv_dtype=dt, outlier_frac=frac, key_mode=mode, seed=5)
+    kt = t[None].cuda()
+    for a, b in ((0, 37), (37, 650), (650, n)):  # blocks from the ring, the tensor and both
+        ctx.append(0, kt[:, a:b], kt[:, a:b])
+    assert ctx.status() == 0
+    x = t.float().numpy()
+    for blk in range(ctx.lengths(0, 0)[1] // S):
+        want = orc.encode_keys(x[blk * S:(blk + 1) * S].transpose(1, 0, 2), frac, mode)
+        got = ctx.export_block(0, 0, blk)
+        assert np.array_equal(got["nf4_scale"][0].view(np.uint32), want["scale"].view(np.uint32))
+        assert np.array_equal(got["nf4_mean"][0], want["mean"])
+        assert np.array_equal(got["key_indices"], orc.pack_key_codes(want["codes"]))
+        if k:
+            assert np.array_equal(got["outlier_idx"], want["out_idx"])
+            assert np.array_equal(got["outlier_val"].view(np.uint16), want["out_val"].view(np.uint16))

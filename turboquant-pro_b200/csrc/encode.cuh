@@ -1,0 +1,88 @@
+// Shared by the encoder kernels of the append path: their arguments, where a token's row is
+// found, packed 16-bit helpers.
+#pragma once
+
+#include "common.cuh"
+
+struct EncodeArgs {
+  tq_geom g;
+  uint8_t* pages;
+  void* hot_k;
+  void* hot_v;
+  uint32_t* pool_dec;
+  uint16_t* pool_val;
+  PageMeta* page_meta;
+  int32_t* seq_len;      // [L][B]
+  uint32_t* pool_cursor; // [L][B][H]
+  int32_t* status;
+  const Tables* tables;
+  const float* bias_means;  // given key zero-points [max_blocks][H][D], or null
+  const void* k;
+  const void* v;
+  int layer, seq_begin, seq_count, n_tokens, max_new_blocks;
+  int64_t seq_stride, tok_stride, head_stride;
+  // PolarQuant keys (TQ_KEYS_POLAR): the value encoder also runs over the keys, writing their
+  // codes where the per-channel codes would go and their norms over the scale / mean arrays
+  int polar_keys_pass;
+};
+
+// Where token `pos` of (seq, head) currently lives: positions below n0 are already in the
+// hot ring, the rest are in the caller's tensor.
+template <int DT>
+struct TokenSource {
+  const void* ring;
+  const void* in;
+  int n0, cap;
+  int64_t tok_stride;
+  // one load from a selected address (no branch: loads of several positions can then be
+  // in flight together)
+  TQ_DEV float ld(int pos, int d) const {
+    const bool old = pos < n0;
+    const void* base = old ? ring : in;
+    const size_t idx =
+        old ? (size_t)(pos % cap) * TQ_D + d : (size_t)(pos - n0) * tok_stride + d;
+    return Elem<DT>::ld(base, idx);
+  }
+};
+
+template <int DT>
+TQ_DEV TokenSource<DT> make_source(const EncodeArgs& a, const void* ring_base, const void* in_base,
+                                   int seq, int head, int n0) {
+  TokenSource<DT> s;
+  s.ring = (const uint8_t*)ring_base +
+           hot_offset_elems(a.g, a.layer, seq, head) * sizeof(typename Elem<DT>::type);
+  s.in = (const uint8_t*)in_base +
+         ((size_t)(seq - a.seq_begin) * a.seq_stride + (size_t)head * a.head_stride) *
+             sizeof(typename Elem<DT>::type);
+  s.n0 = n0;
+  s.cap = a.g.hot_cap;
+  s.tok_stride = a.tok_stride;
+  return s;
+}
+
+// Packed minimum / maximum of two 16-bit floats (fp16 or bf16 by BF): the statistics of two
+// tokens of a channel in one instruction.  The values are the tokens themselves, so nothing
+// is rounded.
+template <bool BF>
+TQ_DEV uint32_t max2_16(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (BF) asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <bool BF>
+TQ_DEV uint32_t min2_16(uint32_t a, uint32_t b) {
+  uint32_t r;
+  if (BF) asm("min.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  else asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <bool BF>
+TQ_DEV float f16bits_to_float(uint32_t h) {
+  return BF ? __uint_as_float(h << 16) : __half2float(__ushort_as_half((unsigned short)h));
+}
+
+// Key encoder for 256-token blocks with up to eight outliers per channel (encode_keys.cu), and
+// whether a geometry is of that form.
+bool tq_keys_block_form(const tq_geom& g);
+int tq_launch_encode_keys_block(const EncodeArgs& a, int device, cudaStream_t st);
