@@ -249,6 +249,15 @@ int32_t tq_xchg_status(tq_xchg* x, int32_t* status, void* stream);
 int32_t tq_dequant_range(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t start, int32_t end,
                          float* k_out, float* v_out, void* stream);
 
+/* The first n_tokens tokens of one sequence, dequantised as by tq_dequant_range, rounded to `dtype`
+ * (TQ_F32, TQ_F16 or TQ_BF16) and written to the rows of an engine's paged tensors: token t goes to
+ * row t % page_tokens of page page_ids[t / page_tokens] (device array; the caller vouches that every
+ * id names a page).  Strides in elements; a row's channels are contiguous. */
+int32_t tq_dequant_paged(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t n_tokens, void* k_pages,
+                         void* v_pages, int32_t dtype, const int64_t* page_ids,
+                         int32_t page_tokens, int64_t page_stride, int64_t row_stride,
+                         int64_t head_stride, void* stream);
+
 /* Copies cold block `block` of (layer, seq) to HOST arrays in the reference's container
  * layout (CompressedPerChannelKV, per_channel_kv.py:103-143; CompressedKV,
  * core.py:96-136) for all KV heads: key_indices [H*S*D/2] (bit-reversed nibbles of

@@ -174,15 +174,32 @@ class DeviceBlockStore:
         restored (0 on a miss)."""
         import torch
 
-        got = self.load(request_id, layer_name)
-        if got is None:
+        layer = self.layer_index(layer_name)
+        ctx = self.ctx
+        slot = self._slot_of(request_id, create=False)
+        n = ctx.lengths(layer, slot)[0] if slot is not None else 0
+        if n == 0:
+            self.counters["misses"] += 1
             return 0
-        k, v = got
-        n = k.shape[1]
+        self.counters["loads"] += 1
+        self.counters["hits"] += 1
         bs = kv_layer.shape[2]
         ids = torch.as_tensor(block_table, device=kv_layer.device, dtype=torch.long).reshape(-1)
         if ids.numel() * bs < n:
             raise ValueError("the block table is too short for the stored prefix")
+        g = ctx.geom
+        if kv_layer.dim() == 5 and kv_layer.device == ctx.device and kv_layer.stride(4) == 1 \
+                and tuple(kv_layer.shape[3:]) == (g.n_kv_heads, g.head_dim) \
+                and kv_layer.dtype in (torch.float32, torch.float16, torch.bfloat16) \
+                and type(kv_layer) is torch.Tensor and not kv_layer.requires_grad:
+            # straight from the codes to the engine's rows; the lookup refuses ids outside the
+            # tensor (and counts negative ones from its end) as indexing the pages would
+            pages = torch.arange(kv_layer.shape[1], device=kv_layer.device)[ids[:-(-n // bs)]]
+            ctx.dequant_into_pages(layer, slot, n, kv_layer[0], kv_layer[1], pages)
+            if not kv_layer.is_inference():  # (an inference tensor keeps no version)
+                torch.autograd.graph.increment_version(kv_layer)
+            return n
+        k, v = ctx.dequant(layer, slot, 0, n)
         pos = torch.arange(n, device=kv_layer.device)
         blk, row = ids[pos // bs], pos % bs
         kv_layer[0][blk, row] = k.permute(1, 0, 2).to(kv_layer.dtype)

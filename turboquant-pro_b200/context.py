@@ -341,6 +341,28 @@ class KVContext:
                                              v.data_ptr() if values else None, self._stream()))
         return k, v
 
+    def dequant_into_pages(self, layer: int, seq: int, n_tokens: int, k_pages, v_pages, ids) -> None:
+        """Writes the first ``n_tokens`` dequantised tokens into an engine's pages: token ``t`` to
+        row ``t % page_tokens`` of page ``ids[t // page_tokens]`` of ``k_pages`` / ``v_pages``
+        ``[n_pages, page_tokens, n_kv_heads, D]`` (one element type and layout, channels
+        contiguous; float32, float16 or bfloat16).  ``ids`` is an int64 CUDA tensor whose entries
+        the caller has checked."""
+        g = self.geom
+        if k_pages.shape != v_pages.shape or k_pages.stride() != v_pages.stride() \
+                or k_pages.dtype != v_pages.dtype or k_pages.device != self.device \
+                or v_pages.device != self.device or k_pages.dim() != 4 or k_pages.stride(3) != 1 \
+                or tuple(k_pages.shape[2:]) != (g.n_kv_heads, g.head_dim):
+            raise ValueError("k_pages and v_pages must share layout, type and device, with "
+                             f"contiguous channels and shape [*, *, {g.n_kv_heads}, {g.head_dim}]")
+        if ids.numel() * k_pages.shape[1] < n_tokens or ids.dtype != _torch().long \
+                or ids.device != self.device or not ids.is_contiguous():
+            raise ValueError("ids must be a contiguous int64 CUDA tensor that covers n_tokens")
+        with _torch().cuda.device(self.device):
+            check(self._lib.tq_dequant_paged(
+                self._h, layer, seq, n_tokens, k_pages.data_ptr(), v_pages.data_ptr(),
+                _dtype_code(k_pages.dtype), ids.data_ptr(), k_pages.shape[1], k_pages.stride(0),
+                k_pages.stride(1), k_pages.stride(2), self._stream()))
+
     def export_block(self, layer: int, seq: int, block: int) -> dict:
         """Cold block ``block`` in the reference's container layout (host numpy arrays):
         the fields of ``CompressedPerChannelKV`` and ``CompressedKV``."""

@@ -251,5 +251,9 @@ int tq_launch_lse_combine(const float* mlo, int n_parts, int n_rows, int head_di
                           cudaStream_t st);
 int tq_launch_dequant(tq_ctx* ctx, int layer, int seq, int start, int end, float* k_out,
                       float* v_out, cudaStream_t st);
+int tq_launch_dequant_paged(tq_ctx* ctx, int layer, int seq, int n_tokens, void* k_pages,
+                            void* v_pages, int dtype, const int64_t* page_ids, int page_tokens,
+                            int64_t page_stride, int64_t row_stride, int64_t head_stride,
+                            cudaStream_t st);
 size_t tq_mma_scratch_bytes(const tq_geom& g, size_t units);
 int tq_launch_clear(tq_ctx* ctx, int layer, int seq_begin, int seq_count, cudaStream_t st);

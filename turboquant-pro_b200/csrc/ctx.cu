@@ -404,6 +404,24 @@ int32_t tq_dequant_range(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t start,
   return tq_launch_dequant(ctx, layer, seq, start, end, k_out, v_out, (cudaStream_t)stream);
 }
 
+int32_t tq_dequant_paged(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t n_tokens, void* k_pages,
+                         void* v_pages, int32_t dtype, const int64_t* page_ids,
+                         int32_t page_tokens, int64_t page_stride, int64_t row_stride,
+                         int64_t head_stride, void* stream) {
+  TQ_REQUIRE(good_ctx(ctx, layer), TQ_ERR_INVALID, "bad context or layer");
+  TQ_REQUIRE(seq >= 0 && seq < ctx->g.n_seqs, TQ_ERR_INVALID, "bad sequence");
+  int n = ctx->len[(size_t)layer * ctx->g.n_seqs + seq];
+  TQ_REQUIRE(n_tokens >= 0 && n_tokens <= n, TQ_ERR_INVALID, "token range out of bounds");
+  TQ_REQUIRE(dtype == TQ_F32 || dtype == TQ_F16 || dtype == TQ_BF16, TQ_ERR_INVALID, "bad dtype");
+  TQ_REQUIRE(page_tokens >= 1, TQ_ERR_INVALID, "page_tokens must be positive");
+  if (n_tokens == 0 || (k_pages == nullptr && v_pages == nullptr)) return TQ_OK;
+  TQ_REQUIRE(page_ids != nullptr, TQ_ERR_INVALID, "page_ids must be a device pointer");
+  TQ_CUDA(cudaSetDevice(ctx->device));
+  return tq_launch_dequant_paged(ctx, layer, seq, n_tokens, k_pages, v_pages, dtype, page_ids,
+                                 page_tokens, page_stride, row_stride, head_stride,
+                                 (cudaStream_t)stream);
+}
+
 int32_t tq_seq_lengths(const tq_ctx* ctx, int32_t layer, int32_t seq, int32_t* total,
                        int32_t* cold, int32_t* hot) {
   TQ_REQUIRE(good_ctx(ctx, layer), TQ_ERR_INVALID, "bad context or layer");
