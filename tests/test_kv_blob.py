@@ -138,3 +138,43 @@ def test_parsed_blob_gives_back_the_container_arrays():
     assert np.array_equal(back["nf4_mean"], want["nf4_mean"])
     sym = blob_to_block(block_to_blob(want, key_mode="nf4"))
     assert not block_from_parsed(sym, key_mode="nf4")["nf4_mean"].any()
+
+
+def test_archive_is_what_numpy_writes_and_other_archives_are_numpy_s_to_read():
+    from turboquant_pro_b200 import kv_blob
+
+    g = load_golden("blob_ref.npz")
+    blk = _oracle_block(g)
+    rng = np.random.default_rng(0)
+    arrays = {"__header__": np.frombuffer(b"{}", np.uint8), "k.a": np.zeros((0,), np.int32),
+              "k.b": rng.standard_normal((1, 3, 128)).astype(np.float32), "v.c": np.float16(2.0).reshape(()),
+              "v.d": np.arange(7, dtype=np.int64), "v.e": np.ones((2, 5), bool)}
+    buf = io.BytesIO()
+    np.savez(buf, **arrays)
+    assert kv_blob._write_npz(arrays) == buf.getvalue()
+    back = kv_blob._read_npz(buf.getvalue(), 1 << 20)
+    assert list(back) == list(arrays)
+    for name, a in arrays.items():
+        assert back[name].dtype == a.dtype and back[name].shape == a.shape
+        assert np.array_equal(back[name], a) and back[name].flags.writeable
+    # another layout of the same members: numpy reads it
+    buf = io.BytesIO()
+    np.savez_compressed(buf, **arrays)
+    assert kv_blob._read_npz(buf.getvalue(), 1 << 20) is None
+    fortran = io.BytesIO()
+    np.savez(fortran, **{"k.f": np.asfortranarray(arrays["k.b"].reshape(3, 128))})
+    assert kv_blob._read_npz(fortran.getvalue(), 1 << 20) is None
+    # damage of any byte of a small archive is never read as something else
+    blob = block_to_blob(blk)
+    whole = kv_blob._read_npz(blob, 1 << 20)
+    assert whole is not None
+    for i in rng.integers(0, len(blob), 300):
+        bad = bytearray(blob)
+        bad[i] ^= 0x41
+        got = kv_blob._read_npz(bytes(bad), 1 << 20)
+        assert got is None or all(np.array_equal(got[n].view(np.uint8), whole[n].view(np.uint8))
+                                  for n in whole), i
+    for n in (0, 10, 22, len(blob) // 2, len(blob) - 1):
+        assert kv_blob._read_npz(blob[:n], 1 << 20) is None
+    with pytest.raises(Exception):
+        blob_to_block(blob[:-1])

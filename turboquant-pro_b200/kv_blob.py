@@ -14,8 +14,14 @@ takes, so a stored block goes into device pages without passing through dense te
 
 from __future__ import annotations
 
+import contextlib
+import functools
 import io
 import json
+import math
+import re
+import struct
+import zlib
 
 import numpy as np
 
@@ -86,10 +92,107 @@ def block_to_blob(block: dict, *, key_mode: str = "nf4_asym", zero_point: str = 
     header = {"codec": CODEC, "shape": list(shape), "dtype": str(dtype),
               "num_tokens": shape[2], "head_dim": shape[3], "n_heads": shape[1],
               "key_scalars": k_sc, "value_scalars": v_sc}
+    return _write_npz({"__header__": np.frombuffer(json.dumps(header).encode(), dtype=np.uint8),
+                       **{f"k.{n}": a for n, a in k_arr.items()},
+                       **{f"v.{n}": a for n, a in v_arr.items()}})
+
+
+# ---- the archive ---------------------------------------------------------------------------
+# A blob is what np.savez writes: a zip archive of stored (uncompressed) .npy members.  zipfile and
+# the .npy header parser spend several times longer on the nine small headers of a block than the
+# checksums and copies of its 280 KB take, so the plain form is written and read here by the record
+# layouts of the zip format (PKWARE's APPNOTE, 4.3); everything else is left to numpy.
+_LOCAL = struct.Struct("<4s5H3L2H")       # local file header
+_CENTRAL = struct.Struct("<4s6H3L5H2L")   # central directory entry
+_END = struct.Struct("<4s4H2LH")          # end of central directory
+_ZIP64 = struct.Struct("<2H2Q")           # extra field with 64-bit sizes
+_NPY = re.compile(rb"\{'descr': '([<|][a-z][0-9]+)', 'fortran_order': False, "
+                  rb"'shape': \(((?:[0-9]+,(?: [0-9]+,)*(?: [0-9]+)?)?)\), \} *\n")
+
+
+@functools.lru_cache(maxsize=256)
+def _npy_header(descr: str, shape: tuple) -> bytes:
     buf = io.BytesIO()
-    np.savez(buf, __header__=np.frombuffer(json.dumps(header).encode(), dtype=np.uint8),
-             **{f"k.{n}": a for n, a in k_arr.items()}, **{f"v.{n}": a for n, a in v_arr.items()})
+    np.lib.format.write_array_header_1_0(
+        buf, {"descr": descr, "fortran_order": False, "shape": shape})
     return buf.getvalue()
+
+
+def _write_npz(arrays: dict) -> bytes:
+    """The bytes np.savez writes for these arrays."""
+    if any(a.dtype.hasobject or not a.flags.c_contiguous for a in arrays.values()) \
+            or sum(a.nbytes for a in arrays.values()) >= 1 << 30:
+        buf = io.BytesIO()
+        np.savez(buf, **arrays)
+        return buf.getvalue()
+    out, central, at = [], [], 0
+    for name, a in arrays.items():
+        file = (name + ".npy").encode("ascii")
+        head = _npy_header(a.dtype.str, a.shape)
+        data = a.reshape(-1).view(np.uint8) if a.size else b""
+        crc = zlib.crc32(data, zlib.crc32(head))
+        size = len(head) + a.nbytes
+        # version 4.5 (64-bit sizes in the extra field), stored, dated 1980-01-01
+        local = _LOCAL.pack(b"PK\3\4", 45, 0, 0, 0, 33, crc, 0xFFFFFFFF, 0xFFFFFFFF, len(file), 20)
+        out += [local, file, _ZIP64.pack(1, 16, size, size), head, data]
+        # (written on a Unix system, readable and writable by the owner)
+        central += [_CENTRAL.pack(b"PK\1\2", 3 << 8 | 45, 45, 0, 0, 0, 33, crc, size, size,
+                                  len(file), 0, 0, 0, 0, 0o600 << 16, at), file]
+        at += _LOCAL.size + len(file) + _ZIP64.size + size
+    n_central = sum(len(c) for c in central)
+    end = _END.pack(b"PK\5\6", 0, 0, len(arrays), len(arrays), n_central, at, 0)
+    return b"".join(out + central + [end])
+
+
+def _read_npz(blob: bytes, max_bytes: int):
+    """The members of an archive of the plain form above, ``{name: array}``; ``None`` for any other
+    one (and for one that is damaged): numpy then reads it, or says what is wrong."""
+    if len(blob) < _END.size:
+        return None
+    end = len(blob) - _END.size
+    sig, disk, disk_c, here, total, n_central, first, comment = _END.unpack_from(blob, end)
+    if sig != b"PK\5\6" or disk or disk_c or here != total or comment or first + n_central != end:
+        return None
+    view, members, at, used = memoryview(blob), {}, first, 0
+    for _ in range(total):
+        if at + _CENTRAL.size > end:
+            return None
+        (sig, _, _, flags, method, _, _, crc, packed, size, n_file, n_extra, n_comment, _, _, _,
+         local) = _CENTRAL.unpack_from(blob, at)
+        file = bytes(view[at + _CENTRAL.size:at + _CENTRAL.size + n_file])
+        at += _CENTRAL.size + n_file
+        if sig != b"PK\1\2" or flags or method or packed != size or size == 0xFFFFFFFF or n_extra \
+                or n_comment or not file.isascii() or not file.endswith(b".npy") or at > end \
+                or local + _LOCAL.size > first:
+            return None
+        (sig, _, flags, method, _, _, crc_l, _, _, n_file_l, n_extra_l) = _LOCAL.unpack_from(blob, local)
+        start = local + _LOCAL.size
+        if sig != b"PK\3\4" or flags or method or crc_l != crc \
+                or bytes(view[start:start + n_file_l]) != file:
+            return None
+        start += n_file_l + n_extra_l
+        if start + size > first or size < 10:
+            return None
+        data = view[start:start + size]
+        n_head = int.from_bytes(data[8:10], "little")
+        if bytes(data[:8]) != b"\x93NUMPY\x01\x00" or 10 + n_head > size or zlib.crc32(data) != crc:
+            return None
+        head = _NPY.fullmatch(bytes(data[10:10 + n_head]))
+        if head is None:
+            return None
+        shape = tuple(int(x) for x in head[2].split(b",") if x.strip())
+        try:
+            dtype = np.dtype(head[1].decode())
+        except TypeError:
+            return None
+        if dtype.hasobject or dtype.itemsize * math.prod(shape) != size - 10 - n_head:
+            return None
+        name = file[:-4].decode()
+        used += size
+        if name in members or used > max_bytes:
+            return None
+        members[name] = np.frombuffer(data[10 + n_head:], dtype=dtype).reshape(shape).copy()
+    return members if at == end else None
 
 
 def _scalars(d: dict) -> dict:
@@ -113,8 +216,11 @@ def blob_to_block(blob: bytes, max_bytes: int = 1 << 30) -> dict:
     """
     if len(blob) > max_bytes:
         raise ValueError(f"blob exceeds max_bytes ({len(blob)} > {max_bytes})")
-    with np.load(io.BytesIO(blob), allow_pickle=False) as z:
-        if "__header__" not in z.files:
+    members = _read_npz(blob, max_bytes)
+    with contextlib.nullcontext(members) if members is not None else \
+            np.load(io.BytesIO(blob), allow_pickle=False) as z:
+        names = list(z) if members is not None else z.files
+        if "__header__" not in names:
             raise ValueError("not a KV block blob: no header")
         header = json.loads(bytes(z["__header__"]).decode())
         if header.get("codec") != CODEC:
@@ -122,7 +228,7 @@ def blob_to_block(blob: bytes, max_bytes: int = 1 << 30) -> dict:
                              f"handles {CODEC!r} only")
         total = 0
         key, value = {}, {}
-        for name in z.files:
+        for name in names:
             if name == "__header__":
                 continue
             a = z[name]
