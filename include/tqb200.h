@@ -287,6 +287,25 @@ int32_t tq_import_block(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t block,
                         int32_t n_outliers, const uint8_t* value_indices,
                         const float* value_norms, void* stream);
 
+/* The batched forms of tq_export_block / tq_import_block: `n_blocks` consecutive blocks of one
+ * sequence converted on the device, between the pages and a staging buffer (device memory of the
+ * caller, 16-byte aligned) whose layout tq_wire_parts gives: byte offsets, inside a block, of the
+ * key codes, key scales, key means, value codes and value norms (the arrays of tq_export_block), and
+ * the bytes of a block.  Outliers of all blocks follow one another (flat indices of their block,
+ * ascending).  tq_outlier_counts reads how many every block holds (host array; synchronises).
+ * tq_import_blocks wants the outliers' start of every (block, head) in `first`
+ * [n_blocks * H + 1] and a device word `short_flag`, and synchronises; the caller has checked that
+ * the indices ascend inside their block and agree with `first`. */
+int32_t tq_wire_parts(const tq_geom* g, int64_t* offsets /* [6] */);
+int32_t tq_outlier_counts(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t block, int32_t n_blocks,
+                          int32_t* counts, void* stream);
+int32_t tq_export_blocks(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t block, int32_t n_blocks,
+                         void* staging, int32_t* outlier_idx, uint16_t* outlier_val,
+                         int64_t n_outliers, void* stream);
+int32_t tq_import_blocks(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t block, int32_t n_blocks,
+                         void* staging, const int32_t* outlier_idx, const uint16_t* outlier_val,
+                         const int32_t* first, int32_t* short_flag, void* stream);
+
 /* Completes a restore: (layer, seq) holds `n_tokens` tokens, of which the cold blocks were
  * imported with tq_import_block and the newest n_tokens - 256 * n_cold_blocks are given here
  * as DEVICE arrays hot_k / hot_v [tokens][n_kv_heads][128] of the context's K/V dtype, with

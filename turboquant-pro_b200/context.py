@@ -21,6 +21,10 @@ import numpy as np
 from . import _lib
 from ._lib import REGIONS, TqBuffers, TqGeom, TqSizes, check
 
+# Blocks converted and copied at a time when a cache is exported or imported: a few tens of MB of
+# staging, and few enough launches that their cost does not show.
+_WIRE_CHUNK = 64
+
 # Lloyd-Max centroids of N(0, 1) for 3 and 4 bits — the direction codebook of the value
 # quantiser (turboquant_pro/core.py:70-93).
 _LLOYD_MAX = {
@@ -398,6 +402,55 @@ class KVContext:
             "shape": (1, h, s, d), "key_bits": g.key_bits, "value_bits": g.value_bits,
         }
 
+    def _wire_parts(self):
+        off = (C.c_int64 * 6)()
+        check(self._lib.tq_wire_parts(C.byref(self.geom), off))
+        return list(off)
+
+    def _export_blocks(self, layer: int, seq: int, block: int, n: int) -> list:
+        """Blocks ``block .. block + n - 1`` as :meth:`export_block` gives them (views of one
+        host buffer): converted on the device and fetched in one copy."""
+        torch = _torch()
+        g = self.geom
+        h, s, d = g.n_kv_heads, g.block_tokens, g.head_dim
+        polar, has = self.key_mode == "polar", g.outlier_k > 0
+        key, scale, mean, val, norm, size = self._wire_parts()
+        counts = np.zeros(n, np.int32)
+        with torch.cuda.device(self.device):
+            check(self._lib.tq_outlier_counts(self._h, layer, seq, block, n, counts.ctypes.data,
+                                              self._stream()))
+            total = int(counts.sum())
+            staging = torch.empty(n * size + 6 * total, dtype=torch.uint8, device=self.device)
+            base = staging.data_ptr()
+            check(self._lib.tq_export_blocks(self._h, layer, seq, block, n, base,
+                                             base + n * size, base + n * size + 4 * total, total,
+                                             self._stream()))
+            raw = staging.cpu().numpy()
+        oidx = raw[n * size:n * size + 4 * total].view(np.int32)
+        oval = raw[n * size + 4 * total:].view(np.float16)
+        out, at = [], 0
+        for i in range(n):
+            part = raw[i * size:(i + 1) * size]
+            m = int(counts[i])
+            blk = {
+                "value_indices": part[val:norm],
+                "value_norms": part[norm:norm + 4 * h * s].view(np.float32).reshape(1, h, s),
+                "shape": (1, h, s, d), "key_bits": g.key_bits, "value_bits": g.value_bits,
+            }
+            if polar:
+                blk.update(key_indices=part[:h * s * d * g.key_bits // 8],
+                           key_norms=part[scale:scale + 4 * h * s].view(np.float32).reshape(1, h, s),
+                           nf4_scale=None, nf4_mean=None, outlier_idx=None, outlier_val=None)
+            else:
+                blk.update(key_indices=part[:h * s * d // 2],
+                           nf4_scale=part[scale:mean].view(np.float32).reshape(1, h, d),
+                           nf4_mean=part[mean:val].view(np.float32).reshape(1, h, d),
+                           outlier_idx=oidx[at:at + m] if has else None,
+                           outlier_val=oval[at:at + m] if has else None)
+            at += m
+            out.append(blk)
+        return out
+
     def export_blob(self, layer: int, seq: int, block: int, rope_theta: float | None = None,
                     zero_point: str = "calibrated") -> bytes:
         """Cold block ``block`` as one ``tqp-kv-npz/1`` byte string, the layout of the
@@ -405,10 +458,13 @@ class KVContext:
         :mod:`turboquant_pro_b200.kv_blob`.  ``zero_point`` / ``rope_theta`` name the key
         zero-point mode the context was set up with (``"sparse"`` after
         :meth:`set_key_mean_mask`, ``"bias"`` after :meth:`set_key_bias_means`)."""
+        return self._to_blob(self.export_block(layer, seq, block), block, rope_theta, zero_point)
+
+    def _to_blob(self, blk: dict, block: int, rope_theta, zero_point) -> bytes:
         from .kv_blob import block_to_blob
 
         dt = {0: "float32", 1: "float16", 2: "bfloat16"}[self.geom.kv_dtype]
-        return block_to_blob(self.export_block(layer, seq, block), key_mode=self.key_mode,
+        return block_to_blob(blk, key_mode=self.key_mode,
                              zero_point=zero_point, mean_mask=self.key_mean_mask,
                              rope_theta=rope_theta,
                              position_start=block * self.geom.block_tokens, dtype=dt)
@@ -417,6 +473,19 @@ class KVContext:
         """The inverse of :meth:`export_block`: writes cold block ``block`` of a cleared cache
         from the container arrays (``nf4_mean`` is the full ``(1, H, D)`` zero-point).
         :meth:`restore_hot` then sets the length."""
+        g = self.geom
+        key_idx, scale, mean, val_idx, norms, oidx, oval = self._block_arrays(blk)
+        n_out = int(oidx.size)
+        with _torch().cuda.device(self.device):
+            check(self._lib.tq_import_block(
+                self._h, layer, seq, block, key_idx.ctypes.data, scale.ctypes.data,
+                mean.ctypes.data, oidx.ctypes.data if n_out else None,
+                oval.ctypes.data if n_out else None, n_out, val_idx.ctypes.data,
+                norms.ctypes.data, self._stream()))
+
+    def _block_arrays(self, blk: dict):
+        """A block's container arrays, flat and checked: key codes, scales, means, value codes,
+        norms, outlier indices and values (as words)."""
         g = self.geom
         h, s, d = g.n_kv_heads, g.block_tokens, g.head_dim
         key_idx = np.ascontiguousarray(blk["key_indices"], dtype=np.uint8).reshape(-1)
@@ -429,19 +498,52 @@ class KVContext:
             raise ValueError("container arrays do not match this context's block shape "
                              f"(H={h}, S={s}, D={d}, value_bits={g.value_bits})")
         oidx = blk.get("outlier_idx")
-        n_out = 0
-        if oidx is not None and len(oidx):
-            oidx = np.ascontiguousarray(oidx, dtype=np.int32)
-            oval = np.ascontiguousarray(blk["outlier_val"]).view(np.uint16).reshape(-1)
-            if oval.size != oidx.size:
-                raise ValueError("outlier_idx and outlier_val differ in length")
-            n_out = int(oidx.size)
-        with _torch().cuda.device(self.device):
-            check(self._lib.tq_import_block(
-                self._h, layer, seq, block, key_idx.ctypes.data, scale.ctypes.data,
-                mean.ctypes.data, oidx.ctypes.data if n_out else None,
-                oval.ctypes.data if n_out else None, n_out, val_idx.ctypes.data,
-                norms.ctypes.data, self._stream()))
+        if oidx is None or not len(oidx):
+            return (key_idx, scale, mean, val_idx, norms, np.empty(0, np.int32),
+                    np.empty(0, np.uint16))
+        oidx = np.ascontiguousarray(oidx, dtype=np.int32).reshape(-1)
+        oval = np.ascontiguousarray(blk["outlier_val"]).view(np.uint16).reshape(-1)
+        if oval.size != oidx.size:
+            raise ValueError("outlier_idx and outlier_val differ in length")
+        return key_idx, scale, mean, val_idx, norms, oidx, oval
+
+    def _import_blocks(self, layer: int, seq: int, block: int, blks: list) -> None:
+        """:meth:`import_block` of consecutive blocks: their containers travel in one copy and are
+        converted on the device."""
+        torch = _torch()
+        g = self.geom
+        h, s, d, n = g.n_kv_heads, g.block_tokens, g.head_dim, len(blks)
+        key, scale, mean, val, norm, size = self._wire_parts()
+        arrays = [self._block_arrays(b) for b in blks]
+        total = sum(a[5].size for a in arrays)
+        # staging | outlier indices | (block, head) starts | flag | outlier values
+        at_first, at_val = n * size + 4 * total, n * size + 4 * total + 4 * (n * h + 2)
+        raw = np.empty(at_val + 2 * total, np.uint8)
+        idx = raw[n * size:at_first].view(np.int32)
+        first = raw[at_first:at_first + 4 * (n * h + 1)].view(np.int32)
+        words = raw[at_val:].view(np.uint16)
+        heads, at = np.arange(h) * (s * d), 0
+        for i, (k_a, s_a, m_a, v_a, n_a, oi, ov) in enumerate(arrays):
+            part = raw[i * size:(i + 1) * size]
+            part[key:key + k_a.size] = k_a
+            part[scale:mean].view(np.float32)[:] = s_a
+            part[mean:val].view(np.float32)[:] = m_a
+            part[val:norm] = v_a
+            part[norm:norm + 4 * n_a.size].view(np.float32)[:] = n_a
+            if oi.size and (oi[0] < 0 or oi[-1] >= h * s * d
+                            or not bool((oi[1:] > oi[:-1]).all())):
+                raise ValueError("outlier indices must ascend inside the (H, S, D) block")
+            first[i * h:(i + 1) * h] = at + np.searchsorted(oi, heads)
+            idx[at:at + oi.size] = oi
+            words[at:at + oi.size] = ov
+            at += oi.size
+        first[n * h] = at
+        with torch.cuda.device(self.device):
+            dev = torch.from_numpy(raw).to(self.device)
+            base = dev.data_ptr()
+            check(self._lib.tq_import_blocks(
+                self._h, layer, seq, block, n, base, base + n * size, base + at_val,
+                base + at_first, base + at_first + 4 * (n * h + 1), self._stream()))
 
     def restore_hot(self, layer: int, seq: int, n_tokens: int, hot_k, hot_v) -> None:
         """Completes a restore: the cache holds ``n_tokens`` tokens, its cold blocks were
@@ -472,13 +574,16 @@ class KVContext:
         :mod:`turboquant_pro_b200.kv_blob`).  A blob with the ``sparse`` zero-point needs this
         context's channel mask (:meth:`set_key_mean_mask`); one with the ``bias`` zero-point
         stores no means, so ``bias_means`` ``(n_kv_heads, D)`` of this block must be given."""
+        self.import_block(layer, seq, block, self._from_blob(blob, bias_means))
+
+    def _from_blob(self, blob: bytes, bias_means) -> dict:
         from .kv_blob import blob_to_block, block_from_parsed
 
-        parsed = blob_to_block(blob)
-        self.import_block(layer, seq, block, block_from_parsed(
-            parsed, key_mode=self.key_mode, mean_mask=self.key_mean_mask, bias_means=bias_means,
+        return block_from_parsed(
+            blob_to_block(blob), key_mode=self.key_mode, mean_mask=self.key_mean_mask,
+            bias_means=bias_means,
             geom=(self.geom.n_kv_heads, self.geom.block_tokens, self.geom.head_dim,
-                  self.geom.value_bits)))
+                  self.geom.value_bits))
 
     def export_state(self, layer: int, seq: int, rope_theta: float | None = None,
                      zero_point: str = "calibrated") -> dict:
@@ -487,8 +592,11 @@ class KVContext:
         of a context with the same geometry, seed and key format restores it exactly."""
         total, cold, _hot = self.lengths(layer, seq)
         nb = cold // self.geom.block_tokens
-        blocks = [self.export_blob(layer, seq, b, rope_theta=rope_theta, zero_point=zero_point)
-                  for b in range(nb)]
+        blocks = []
+        for b0 in range(0, nb, _WIRE_CHUNK):
+            blks = self._export_blocks(layer, seq, b0, min(_WIRE_CHUNK, nb - b0))
+            blocks += [self._to_blob(blk, b0 + i, rope_theta, zero_point)
+                       for i, blk in enumerate(blks)]
         torch = _torch()
         if total > cold:  # the window's values are stored exactly
             hk, hv = self.dequant(layer, seq, cold, total)
@@ -518,9 +626,10 @@ class KVContext:
         if len(state["blocks"]) != self.cold_blocks(n):
             raise ValueError("block count does not match the token count")
         self.clear(layer, seq)
-        for b, blob in enumerate(state["blocks"]):
-            self.import_blob(layer, seq, b, blob,
-                             bias_means=None if bias_means is None else bias_means[b])
+        for b0 in range(0, len(state["blocks"]), _WIRE_CHUNK):
+            self._import_blocks(layer, seq, b0, [
+                self._from_blob(blob, None if bias_means is None else bias_means[b0 + i])
+                for i, blob in enumerate(state["blocks"][b0:b0 + _WIRE_CHUNK])])
         if n:
             hot = [torch.from_numpy(np.ascontiguousarray(state[name])).view(self.kv_dtype)
                    for name in ("hot_k", "hot_v")]
