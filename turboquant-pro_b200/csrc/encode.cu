@@ -1449,15 +1449,19 @@ __global__ void __launch_bounds__(ENC5_PARTS* TQ_D, 1) encode_values_tc5_kernel(
 
 // ---------------------------------------------------------------------------------------
 // Hot-ring writer: the new tokens that stay uncompressed go to slot (position % hot_cap).
-// grid = (tokens, heads, seqs); token index counts back from the newest.  The CTA that
+// grid = (tokens / RW_TOK, heads, seqs); token index counts back from the newest.  A CTA moves
+// RW_TOK rows of keys and values in 16-byte pieces, all loads before the stores (one row and one
+// atomic a CTA took 40 us for 512 tokens x 8 heads x 8 sequences, bound by the atomics).  The CTA that
 // finishes last then adds the new tokens to the sequence lengths: every kernel of the append
 // (the encoders before this one in the stream, and every CTA of this one) has read the old
 // lengths by then.  The kernel may be launched with programmatic stream serialization: it
 // waits for the kernel before it in the stream before it reads or writes anything.
 // ---------------------------------------------------------------------------------------
+constexpr int RW_TOK = 16;
 template <int DT>
 __global__ void __launch_bounds__(TQ_D) ring_write_kernel(EncodeArgs a) {
   using T = typename Elem<DT>::type;
+  constexpr int EPC = 16 / (int)sizeof(T), CH = TQ_D / EPC, N = RW_TOK * CH / TQ_D;
   const tq_geom& g = a.g;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1465,15 +1469,41 @@ __global__ void __launch_bounds__(TQ_D) ring_write_kernel(EncodeArgs a) {
   const int head = blockIdx.y;
   const int n0 = a.seq_len[a.layer * g.n_seqs + seq];
   const int n1 = n0 + a.n_tokens;
-  const int pos = n1 - 1 - (int)blockIdx.x;
   const int hot_start = n_cold_blocks(n1, g.hot_window, g.block_tokens) * g.block_tokens;
-  if (pos >= n0 && pos >= hot_start) {
-    const size_t in = (size_t)(seq - a.seq_begin) * a.seq_stride +
-                      (size_t)(pos - n0) * a.tok_stride + (size_t)head * a.head_stride + threadIdx.x;
-    const size_t out =
-        hot_offset_elems(g, a.layer, seq, head) + (size_t)(pos % g.hot_cap) * TQ_D + threadIdx.x;
-    ((T*)a.hot_k)[out] = ((const T*)a.k)[in];
-    ((T*)a.hot_v)[out] = ((const T*)a.v)[in];
+  const int first = max(n0, hot_start);  // the oldest token to write
+  const int newest = n1 - 1 - (int)blockIdx.x * RW_TOK;
+  const size_t in0 = (size_t)(seq - a.seq_begin) * a.seq_stride + (size_t)head * a.head_stride;
+  const size_t out0 = hot_offset_elems(g, a.layer, seq, head);
+  const bool aligned = (((uintptr_t)a.k | (uintptr_t)a.v) & 15) == 0 &&
+                       ((a.seq_stride | a.tok_stride | a.head_stride) & (EPC - 1)) == 0;
+  if (aligned) {
+    uint4 kv[2][N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int id = threadIdx.x + TQ_D * i, pos = newest - id / CH;
+      if (pos >= first) {
+        const size_t in = in0 + (size_t)(pos - n0) * a.tok_stride + id % CH * EPC;
+        kv[0][i] = *(const uint4*)((const T*)a.k + in);
+        kv[1][i] = *(const uint4*)((const T*)a.v + in);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int id = threadIdx.x + TQ_D * i, pos = newest - id / CH;
+      if (pos >= first) {
+        const size_t out = out0 + (size_t)(pos % g.hot_cap) * TQ_D + id % CH * EPC;
+        *(uint4*)((T*)a.hot_k + out) = kv[0][i];
+        *(uint4*)((T*)a.hot_v + out) = kv[1][i];
+      }
+    }
+  } else {
+    for (int t = 0; t < RW_TOK && newest - t >= first; ++t) {
+      const int pos = newest - t;
+      const size_t in = in0 + (size_t)(pos - n0) * a.tok_stride + threadIdx.x;
+      const size_t out = out0 + (size_t)(pos % g.hot_cap) * TQ_D + threadIdx.x;
+      ((T*)a.hot_k)[out] = ((const T*)a.k)[in];
+      ((T*)a.hot_v)[out] = ((const T*)a.v)[in];
+    }
   }
   // last CTA out: the counter sits in the status word's 256-byte block and returns to zero
   __shared__ int s_last;
@@ -1569,7 +1599,8 @@ int launch_encode_t(const EncodeArgs& a, int sm_count, int device, cudaStream_t 
   // (launched so that it may be scheduled while the kernel before it in the stream drains; it
   // waits for that kernel itself)
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(a.n_tokens, g.hot_window), g.n_kv_heads, a.seq_count);
+  cfg.gridDim = dim3((std::min(a.n_tokens, g.hot_window) + RW_TOK - 1) / RW_TOK, g.n_kv_heads,
+                     a.seq_count);
   cfg.blockDim = dim3(TQ_D);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
