@@ -7,28 +7,9 @@
 //   s = q.mean + sum_d (q_d * scale_d) * NF4[code_d] + sum_{outliers of the token} q_d * delta_d
 // Value accumulation stays in the rotated code space, acc_e += p * norm * centroid[code_e];
 // the single inverse rotation acc @ Pi is applied once per query head in the combine.
-#include "common.cuh"
+#include "decode_generic.cuh"
 
 namespace {
-
-struct DecodeArgs {
-  tq_geom g;
-  const uint8_t* pages;
-  const void* hot_k;
-  const void* hot_v;
-  const uint32_t* pool_dec;
-  const PageMeta* page_meta;
-  const int32_t* seq_len;
-  const Tables* tables;
-  const void* q;
-  float* partials;  // [units][max_splits][G][2 + D]
-  float* out;       // [n_seqs][n_q_heads][D] or null
-  float* mlo;       // [n_seqs][n_q_heads][2 + D] or null
-  int layer, q_dtype;
-  int ns_cold, ns_hot;
-  int block_begin, block_end, with_hot;
-  float scale;
-};
 
 TQ_DEV float ld_any(const void* p, size_t i, int dt) {
   if (dt == TQ_F32) return ((const float*)p)[i];
@@ -522,6 +503,22 @@ void launch_generic(const DecodeArgs& a, int n_units, cudaStream_t st) {
   decode_generic_kernel<GT><<<grid, WARPS * 32, 0, st>>>(a);
 }
 
+// Groups of five and more on 256-token blocks: decode_pages.cu.  Everything else here.
+void launch_generic_any(const DecodeArgs& a, int n_units, cudaStream_t st) {
+  const tq_geom& g = a.g;
+  if (tq_decode_pages_form(g)) {
+    tq_launch_decode_pages(a, n_units, st);
+    return;
+  }
+  int gt = g.group >= 8 ? 8 : (g.group > 2 ? 4 : (g.group > 1 ? 2 : 1));
+  switch (gt) {
+    case 1: launch_generic<1>(a, n_units, st); break;
+    case 2: launch_generic<2>(a, n_units, st); break;
+    case 4: launch_generic<4>(a, n_units, st); break;
+    default: launch_generic<8>(a, n_units, st); break;
+  }
+}
+
 }  // namespace
 
 struct tq_xchg;
@@ -589,13 +586,7 @@ int tq_launch_decode(tq_ctx* ctx, int layer, const void* q, int q_dtype, int blo
 
   cudaEvent_t e0 = tq_prof_event(ctx, 0), e1 = tq_prof_event(ctx, 1), e2 = tq_prof_event(ctx, 2);
   if (e0) cudaEventRecord(e0, st);
-  int gt = g.group >= 8 ? 8 : (g.group > 2 ? 4 : (g.group > 1 ? 2 : 1));
-  switch (gt) {
-    case 1: launch_generic<1>(a, n_units, st); break;
-    case 2: launch_generic<2>(a, n_units, st); break;
-    case 4: launch_generic<4>(a, n_units, st); break;
-    default: launch_generic<8>(a, n_units, st); break;
-  }
+  launch_generic_any(a, n_units, st);
   if (e1) cudaEventRecord(e1, st);
   combine_kernel<<<dim3(n_units, g.group), TQ_D, 0, st>>>(a);
   if (e2) {
@@ -701,13 +692,7 @@ extern "C" int32_t tq_decode_static_scratch(tq_ctx* ctx, int32_t layer, const vo
   a.ns_cold = ns_cold;
   a.ns_hot = ns_hot;
 
-  int gt = g.group >= 8 ? 8 : (g.group > 2 ? 4 : (g.group > 1 ? 2 : 1));
-  switch (gt) {
-    case 1: launch_generic<1>(a, n_units, st); break;
-    case 2: launch_generic<2>(a, n_units, st); break;
-    case 4: launch_generic<4>(a, n_units, st); break;
-    default: launch_generic<8>(a, n_units, st); break;
-  }
+  launch_generic_any(a, n_units, st);
   combine_kernel<<<dim3(n_units, g.group), TQ_D, 0, st>>>(a);
   ctx->last_launches = 2;
   ctx->last_kernel = TQ_KERNEL_GENERAL;

@@ -1,0 +1,30 @@
+// Arguments shared by the float32 decode kernels (decode_generic.cu, decode_pages.cu).
+#pragma once
+
+#include "common.cuh"
+
+struct DecodeArgs {
+  tq_geom g;
+  const uint8_t* pages;
+  const void* hot_k;
+  const void* hot_v;
+  const uint32_t* pool_dec;
+  const PageMeta* page_meta;
+  const int32_t* seq_len;
+  const Tables* tables;
+  const void* q;
+  float* partials;  // [units][max_splits][G][2 + D]
+  float* out;       // [n_seqs][n_q_heads][D] or null
+  float* mlo;       // [n_seqs][n_q_heads][2 + D] or null
+  int layer, q_dtype;
+  int ns_cold, ns_hot;
+  int block_begin, block_end, with_hot;
+  float scale;
+};
+
+// Query groups of five and more on 256-token blocks (per-channel keys) take the page kernel (at three
+// heads its sums came out a tenth further from 64 bits than the general kernel's; above, no further).
+TQ_HD bool tq_decode_pages_form(const tq_geom& g) {
+  return g.block_tokens == 256 && g.key_mode != TQ_KEYS_POLAR && g.group > 4;
+}
+void tq_launch_decode_pages(const DecodeArgs& a, int n_units, cudaStream_t st);
