@@ -13,13 +13,17 @@ hand-written kernels behind the C ABI (``include/tqb200.h``).
 
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import functools
 import math
 
 import numpy as np
 
 from . import _lib
 from ._lib import REGIONS, TqBuffers, TqGeom, TqSizes, check
+
+_NO_GUARD = contextlib.nullcontext()
 
 # Blocks converted and copied at a time when a cache is exported or imported: a few tens of MB of
 # staging, and few enough launches that their cost does not show.
@@ -60,10 +64,15 @@ def _torch():
     return torch
 
 
-def _dtype_code(torch_dtype) -> int:
+@functools.cache
+def _dtype_codes() -> dict:
     torch = _torch()
     return {torch.float32: _lib.TQ_F32, torch.float16: _lib.TQ_F16,
-            torch.bfloat16: _lib.TQ_BF16}[torch_dtype]
+            torch.bfloat16: _lib.TQ_BF16}
+
+
+def _dtype_code(torch_dtype) -> int:
+    return _dtype_codes()[torch_dtype]
 
 
 def _torch_dtype(name):
@@ -142,7 +151,7 @@ class KVContext:
         self.pi, self.pi_t = pi, pi_t
         self.centroids, self.boundaries = value_codebook(head_dim, value_bits)
         handle = C.c_void_p()
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_ctx_create(
                 C.byref(g), C.byref(bufs), device, pi.ctypes.data, pi_t.ctypes.data,
                 self.centroids.ctypes.data, self.boundaries.ctypes.data,
@@ -153,8 +162,18 @@ class KVContext:
             self.set_key_mean_mask(key_mean_mask)
 
     # -- plumbing --------------------------------------------------------------------
+    # A decode step of a layer is some ten microseconds on the GPU, and so is a call made up of
+    # torch's device guard and a Stream object: both are taken only as far as they are needed.
     def _stream(self):
-        return C.c_void_p(_torch().cuda.current_stream(self.device).cuda_stream)
+        return _torch()._C._cuda_getCurrentRawStream(self.device.index)
+
+    def _here(self):
+        """The device guard of a library call (the library selects its device itself; the guard
+        gives the caller's back), nothing where the context's device is the current one."""
+        cuda = _torch().cuda
+        if cuda.current_device() == self.device.index:
+            return _NO_GUARD
+        return cuda.device(self.device)
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -194,7 +213,6 @@ class KVContext:
         contiguous last dimension) of ``kv_dtype``.  Performs every flush the reference
         would perform for token-by-token appends, with the same block boundaries.
         """
-        torch = _torch()
         if k.dim() != 4 or k.shape != v.shape:
             raise ValueError(f"expected k, v of shape [n_seqs, T, H, D], got {tuple(k.shape)} "
                              f"and {tuple(v.shape)}")
@@ -211,7 +229,7 @@ class KVContext:
         if v.stride() != k.stride():
             v = v.contiguous()
             k = k.contiguous()
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_append(self._h, layer, seq_begin, k.shape[0], k.data_ptr(),
                                       v.data_ptr(), k.shape[1], k.stride(0), k.stride(1),
                                       k.stride(2), self._stream()))
@@ -244,11 +262,10 @@ class KVContext:
         synchronises and raises :class:`TqError` if the kernel reported a wait that ran out
         (status bit 1: the output is then undefined).
         """
-        torch = _torch()
         g = self.geom
         q = self._check_q(q)
         out = self._check_result(out, (g.n_seqs, g.n_q_heads, g.head_dim), "out")
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_decode(self._h, layer, q.data_ptr(), _dtype_code(q.dtype),
                                       out.data_ptr(), self._stream()))
         if check_status:
@@ -269,11 +286,10 @@ class KVContext:
         split-K partials live in a fixed array inside the library (at most 1024
         (sequence, query head) pairs; calls must not overlap on the device).  ``out`` should
         be passed by such callers; it is created here only as a convenience."""
-        torch = _torch()
         g = self.geom
         q = self._check_q(q)
         out = self._check_result(out, (g.n_seqs, g.n_q_heads, g.head_dim), "out")
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_decode_static_scratch(self._h, layer, q.data_ptr(),
                                                      _dtype_code(q.dtype), out.data_ptr(),
                                                      self._stream()))
@@ -283,11 +299,10 @@ class KVContext:
                        mlo=None):
         """Un-normalised ``(m, l, o)`` states over cold blocks ``[block_begin, block_end)``
         (+ the hot window): float32 ``[n_seqs, n_q_heads, 2 + D]``."""
-        torch = _torch()
         g = self.geom
         q = self._check_q(q)
         mlo = self._check_result(mlo, (g.n_seqs, g.n_q_heads, 2 + g.head_dim), "mlo")
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_decode_partial(self._h, layer, q.data_ptr(), _dtype_code(q.dtype),
                                               block_begin, block_end, int(bool(with_hot)),
                                               mlo.data_ptr(), self._stream()))
@@ -302,12 +317,11 @@ class KVContext:
         output.  Raises ``NotImplementedError`` where the layer has no such fused form; the
         two-call form (``decode_partial`` then ``PeerExchange.gather_merge``) works everywhere
         and gives the same bits."""
-        torch = _torch()
         g = self.geom
         q = self._check_q(q)
         out = self._check_result(out, (g.n_seqs, g.n_q_heads, g.head_dim), "out")
         h = getattr(exchange, "_h", exchange)
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_decode_exchange(self._h, layer, q.data_ptr(), _dtype_code(q.dtype),
                                                block_begin, block_end, int(bool(with_hot)), h,
                                                out.data_ptr(), phases, self._stream()))
@@ -323,7 +337,7 @@ class KVContext:
         mlo = mlo.contiguous()
         n_parts, n_rows, w = mlo.shape
         out = self._check_result(out, (n_rows, w - 2), "out")
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_lse_combine(mlo.data_ptr(), n_parts, n_rows, w - 2,
                                            out.data_ptr(), self._stream()))
         return out
@@ -339,7 +353,7 @@ class KVContext:
                         device=self.device) if keys else None
         v = torch.empty((g.n_kv_heads, n, g.head_dim), dtype=torch.float32,
                         device=self.device) if values else None
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_dequant_range(self._h, layer, seq, start, end,
                                              k.data_ptr() if keys else None,
                                              v.data_ptr() if values else None, self._stream()))
@@ -361,7 +375,7 @@ class KVContext:
         if ids.numel() * k_pages.shape[1] < n_tokens or ids.dtype != _torch().long \
                 or ids.device != self.device or not ids.is_contiguous():
             raise ValueError("ids must be a contiguous int64 CUDA tensor that covers n_tokens")
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_dequant_paged(
                 self._h, layer, seq, n_tokens, k_pages.data_ptr(), v_pages.data_ptr(),
                 _dtype_code(k_pages.dtype), ids.data_ptr(), k_pages.shape[1], k_pages.stride(0),
@@ -382,7 +396,7 @@ class KVContext:
         n_out = C.c_int32(0)
         val_idx = np.empty(h * s * d * g.value_bits // 8, np.uint8)
         norms = np.empty((1, h, s), np.float32)
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_export_block(
                 self._h, layer, seq, block, key_idx.ctypes.data, scale.ctypes.data,
                 mean.ctypes.data, oidx.ctypes.data, oval.ctypes.data, cap, C.byref(n_out),
@@ -416,7 +430,7 @@ class KVContext:
         polar, has = self.key_mode == "polar", g.outlier_k > 0
         key, scale, mean, val, norm, size = self._wire_parts()
         counts = np.zeros(n, np.int32)
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_outlier_counts(self._h, layer, seq, block, n, counts.ctypes.data,
                                               self._stream()))
             total = int(counts.sum())
@@ -476,7 +490,7 @@ class KVContext:
         g = self.geom
         key_idx, scale, mean, val_idx, norms, oidx, oval = self._block_arrays(blk)
         n_out = int(oidx.size)
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_import_block(
                 self._h, layer, seq, block, key_idx.ctypes.data, scale.ctypes.data,
                 mean.ctypes.data, oidx.ctypes.data if n_out else None,
@@ -538,7 +552,7 @@ class KVContext:
             words[at:at + oi.size] = ov
             at += oi.size
         first[n * h] = at
-        with torch.cuda.device(self.device):
+        with self._here():
             dev = torch.from_numpy(raw).to(self.device)
             base = dev.data_ptr()
             check(self._lib.tq_import_blocks(
@@ -548,7 +562,6 @@ class KVContext:
     def restore_hot(self, layer: int, seq: int, n_tokens: int, hot_k, hot_v) -> None:
         """Completes a restore: the cache holds ``n_tokens`` tokens, its cold blocks were
         imported, and ``hot_k`` / ``hot_v`` (tensors ``[tokens, n_kv_heads, D]``) are the tokens after the last cold block."""
-        torch = _torch()
         g = self.geom
         n_hot = n_tokens - self.cold_blocks(n_tokens) * g.block_tokens
         for t in (hot_k, hot_v):
@@ -557,7 +570,7 @@ class KVContext:
                                  f"{(n_hot, g.n_kv_heads, g.head_dim)}, got {tuple(t.shape)}")
         k = hot_k.to(device=self.device, dtype=self.kv_dtype).contiguous()
         v = hot_v.to(device=self.device, dtype=self.kv_dtype).contiguous()
-        with torch.cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_restore_hot(self._h, layer, seq, n_tokens, k.data_ptr(),
                                            v.data_ptr(), k.stride(0), k.stride(1),
                                            self._stream()))
@@ -645,20 +658,20 @@ class KVContext:
     def memory_stats(self, layer: int, seq: int):
         """(cold_bytes, hot_bytes) counted like the reference's containers."""
         cold, hot = C.c_double(), C.c_double()
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_memory_stats(self._h, layer, seq, C.byref(cold), C.byref(hot),
                                             self._stream()))
         return cold.value, hot.value
 
     def clear(self, layer: int, seq: int = -1) -> None:
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_clear(self._h, layer, seq, self._stream()))
 
     def status(self) -> int:
         """Device status flags (bit 0: an outlier pool overflowed; bit 1: a bounded wait of the
         tensor-core decode kernel ran out and that call's output is undefined); clears them."""
         f = C.c_int32()
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_status(self._h, C.byref(f), self._stream()))
         return f.value
 
@@ -679,7 +692,7 @@ class KVContext:
             m = np.ascontiguousarray(np.asarray(mask).astype(bool).astype(np.uint8))
             if m.shape != (self.geom.head_dim,):
                 raise ValueError(f"expected a mask of {self.geom.head_dim} channels")
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_set_key_mean_mask(self._h, m.ctypes.data if m is not None else None,
                                                  self._stream()))
         self.key_mean_mask = None if m is None else m.astype(bool)
@@ -696,7 +709,7 @@ class KVContext:
             if m.shape != (g.max_blocks, g.n_kv_heads, g.head_dim):
                 raise ValueError(f"expected means of shape "
                                  f"{(g.max_blocks, g.n_kv_heads, g.head_dim)}, got {m.shape}")
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_set_key_bias_means(
                 self._h, m.ctypes.data if m is not None else None, self._stream()))
 
@@ -719,7 +732,7 @@ class KVContext:
         """Switch the decode kernel's pipeline stamping on/off; with ``read`` return the
         stamps of the last traced decode as a (64, 8) uint64 array of SM clocks."""
         buf = np.zeros((64, 8), np.uint64) if read else None
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_debug_trace(self._h, int(bool(on)),
                                            buf.ctypes.data if read else None, self._stream()))
         return buf
@@ -731,6 +744,6 @@ class KVContext:
     def profile_read(self):
         """(attention-kernel ms, combine-kernel ms, calls) summed since the last read."""
         a, c, n = C.c_double(), C.c_double(), C.c_int32()
-        with _torch().cuda.device(self.device):
+        with self._here():
             check(self._lib.tq_profile_read(self._h, C.byref(a), C.byref(c), C.byref(n)))
         return a.value, c.value, n.value
