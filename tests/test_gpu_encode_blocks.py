@@ -59,3 +59,48 @@ def test_key_blocks_equal_the_oracle(dt, mode, frac, k):
         if k:
             assert np.array_equal(got["outlier_idx"], want["out_idx"])
             assert np.array_equal(got["outlier_val"].view(np.uint16), want["out_val"].view(np.uint16))
+
+
+def _blocks(t, mode, frac, dt):
+    """The exported cold blocks of tokens appended in one go."""
+    from turboquant_pro_b200 import KVContext
+
+    ctx = KVContext(n_layers=1, n_seqs=1, n_kv_heads=H, n_q_heads=H, value_bits=3, hot_window=W,
+                    max_tokens_per_seq=t.shape[0], kv_dtype=dt, outlier_frac=frac, key_mode=mode, seed=5)
+    kt = t[None].cuda()
+    ctx.append(0, kt, kt)
+    assert ctx.status() == 0
+    return [ctx.export_block(0, 0, b) for b in range(ctx.lengths(0, 0)[1] // S)]
+
+
+def _outliers(x, k):
+    """(flat indices, fp16 bits) of a block ``(S, H, 128)``: every token whose magnitude reaches the
+    channel's k-th largest; a NaN is below every magnitude and never one."""
+    mag = np.where(np.isnan(x), -1.0, np.abs(x)).transpose(1, 0, 2)
+    kth = np.sort(mag, axis=1)[:, -k, :]
+    flat = np.flatnonzero((mag >= kth[:, None, :]) & (mag >= 0.0))
+    with np.errstate(over="ignore"):
+        return flat, x.transpose(1, 0, 2).reshape(-1)[flat].astype(np.float16).view(np.uint16)
+
+
+@pytest.mark.parametrize("dt", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("mode", ["nf4_asym", "nf4", "uniform"])
+@pytest.mark.parametrize("frac,k", [(0.003, 1), (0.02, 5), (0.032, 8)])
+def test_nan_keys_are_never_outliers(dt, mode, frac, k):
+    import torch
+
+    n = W + 2 * S
+    x = np.random.default_rng(2).standard_normal((n, H, 128)).astype(np.float32)
+    x[7, 0, 5] = np.nan                       # beside ordinary tokens
+    x[7, 1, :] = np.nan                       # a whole row
+    x[::3, 0, 6] = np.nan
+    x[:, 0, 7] = 0.0                          # the k-th magnitude is zero
+    x[2::5, 0, 7] = np.nan
+    x[:, 1, 8] = np.nan                       # fewer than k numbers
+    x[[3, 90, 300], 1, 8] = [1.0, -2.0, 0.5]
+    t = torch.from_numpy(x).to(getattr(torch, dt))
+    x = t.float().numpy()
+    for blk, got in enumerate(_blocks(t, mode, frac, dt)[:2]):
+        idx, val = _outliers(x[blk * S:(blk + 1) * S], k)
+        assert np.array_equal(got["outlier_idx"], idx)
+        assert np.array_equal(got["outlier_val"].view(np.uint16), val)

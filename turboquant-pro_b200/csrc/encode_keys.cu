@@ -505,18 +505,21 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (the image is read by a bulk copy)
   if (kk > 0) {
     // NSUB threads a channel share the eight tokens of each of its groups; magnitudes as integers
-    // (their bit patterns order like the numbers)
+    // (their bit patterns order like the numbers; a NaN is below all of them and never an outlier)
     constexpr int NSUB = THREADS / TQ_D, PER = 8 / NSUB;
     const int d = tid / NSUB, sub = tid % NSUB;
-    auto mag = [&](int t) -> uint32_t {
-      if constexpr (F32) return ((const uint32_t*)rows)[t * TQ_D + d] & 0x7FFFFFFFu;
-      else return ((const unsigned short*)rows)[t * TQ_D + d] & 0x7FFFu;
+    constexpr int INF_BITS = F32 ? 0x7F800000 : BF ? 0x7F80 : 0x7C00;
+    auto mag = [&](int t) -> int {
+      int m;
+      if constexpr (F32) m = (int)(((const uint32_t*)rows)[t * TQ_D + d] & 0x7FFFFFFFu);
+      else m = ((const unsigned short*)rows)[t * TQ_D + d] & 0x7FFF;
+      return m > INF_BITS ? -1 : m;
     };
     auto token = [&](int gi, int k) -> int { return gi / GPT * NT + gi % GPT + GPT * (sub + NSUB * k); };
-    uint32_t top[EK_K];
+    int top[EK_K];
 #pragma unroll
-    for (int j = 0; j < EK_K; ++j) top[j] = 0u;
-    auto insert = [&](uint32_t v) {
+    for (int j = 0; j < EK_K; ++j) top[j] = 0;
+    auto insert = [&](int v) {
       if (kk > 5) {
 #pragma unroll
         for (int j = 0; j < 3; ++j) top[j] = min(max(v, top[j]), top[j + 1]);
@@ -528,7 +531,7 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     const uint32_t sel = s_groups[d];
     for (uint32_t left = sel; left != 0u; left &= left - 1u) {
       const int gi = __ffs((int)left) - 1;
-      uint32_t v[PER];
+      int v[PER];
 #pragma unroll
       for (int k = 0; k < PER; ++k) v[k] = mag(token(gi, k));
 #pragma unroll
@@ -536,14 +539,14 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     }
 #pragma unroll
     for (int o = 1; o < NSUB; o <<= 1) {  // the threads of a channel merge their lists
-      uint32_t other[EK_K];
+      int other[EK_K];
 #pragma unroll
       for (int j = 0; j < EK_K; ++j) other[j] = __shfl_xor_sync(0xffffffffu, top[j], o);
 #pragma unroll
       for (int j = 0; j < EK_K; ++j)
         if (kk > 5 || j >= 3) insert(other[j]);
     }
-    uint32_t kth = 0u;
+    int kth = 0;
 #pragma unroll
     for (int j = 0; j < EK_K; ++j) kth = j == EK_K - kk ? top[j] : kth;
     // every token's outlier channels as a bit mask
