@@ -66,7 +66,8 @@ def _blocks(t, mode, frac, dt):
     from turboquant_pro_b200 import KVContext
 
     ctx = KVContext(n_layers=1, n_seqs=1, n_kv_heads=H, n_q_heads=H, value_bits=3, hot_window=W,
-                    max_tokens_per_seq=t.shape[0], kv_dtype=dt, outlier_frac=frac, key_mode=mode, seed=5)
+                    max_tokens_per_seq=8 * t.shape[0], kv_dtype=dt, outlier_frac=frac,
+                    key_mode=mode, seed=5)  # (room for many equal magnitudes)
     kt = t[None].cuda()
     ctx.append(0, kt, kt)
     assert ctx.status() == 0
@@ -102,5 +103,48 @@ def test_nan_keys_are_never_outliers(dt, mode, frac, k):
     x = t.float().numpy()
     for blk, got in enumerate(_blocks(t, mode, frac, dt)[:2]):
         idx, val = _outliers(x[blk * S:(blk + 1) * S], k)
+        assert np.array_equal(got["outlier_idx"], idx)
+        assert np.array_equal(got["outlier_val"].view(np.uint16), val)
+
+
+@pytest.mark.parametrize("dt", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("mode", ["nf4_asym", "nf4", "uniform"])
+def test_keys_at_and_beyond_the_top_of_the_range(dt, mode):
+    """Against the general encoder, which takes the same tokens with nine outliers a channel (the
+    codes, scales and zero-points do not depend on their number)."""
+    import torch
+
+    n = W + 2 * S
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((n, H, 128))
+    sign = rng.choice([-1.0, 1.0], n)
+    x[9, 0, 4] = np.inf
+    x[9, 0, 7] = -np.inf
+    x[[9, 30], 0, 10] = [np.inf, -np.inf]
+    x[:, 0, 12] = np.inf * sign
+    x[5, 0, 14] = np.inf
+    x[8, 0, 14] = np.nan
+    x[8, 0, 16] = np.nan
+    x[40, 0, 20] = 3.3e38                        # above the largest border of the table
+    x[40, 0, 23] = -3.3e38
+    x[:, 0, 26] = 3.35e38 * sign
+    x[:, 0, 28] = 2.5e38 * rng.uniform(-1, 1, n)
+    x[:, 0, 31] = 1.0e38 + 1.0e36 * rng.standard_normal(n)
+    x[:, 0, 33] = 3.0e38
+    x[:, 0, 34] = -1.0e38 * rng.uniform(0, 3.3, n)
+    x[:, 0, 36] = 2.0 ** 126 * rng.uniform(0.99, 1.01, n) * sign
+    x[:, 0, 38] = 2.0 ** 125 * rng.uniform(-1, 1, n)
+    x[:, 0, 40] = 6.5e4 * rng.uniform(-1, 1, n)  # (the top of fp16)
+    x[:, 0, 41] = 1.0e-40 * rng.standard_normal(n)
+    with np.errstate(over="ignore"):
+        t = torch.from_numpy(x.astype(np.float32)).to(getattr(torch, dt))
+    x = t.float().numpy()
+    for blk, (got, want) in enumerate(zip(_blocks(t, mode, 0.02, dt)[:2],
+                                          _blocks(t, mode, 0.036, dt)[:2], strict=True)):
+        codes = [b["key_indices"].reshape(H, S, 64) for b in (got, want)]
+        assert not np.argwhere((codes[0] != codes[1]).any(axis=1)).tolist()
+        assert np.array_equal(got["nf4_scale"], want["nf4_scale"])
+        assert np.array_equal(got["nf4_mean"], want["nf4_mean"], equal_nan=True)
+        idx, val = _outliers(x[blk * S:(blk + 1) * S], 5)
         assert np.array_equal(got["outlier_idx"], idx)
         assert np.array_equal(got["outlier_val"].view(np.uint16), val)

@@ -309,10 +309,12 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     // An element closer than this to a border is computed again.  The table holds the border with
     // its four low mantissa bits replaced (at most 8 ulp, 2^-20 of |border| <= |mu| + range) and
     // the reference's levels and distances round by an ulp each: 2^-19 of the sum covers both.
-    // Where the range is tiny against the zero-point the levels themselves round together:
+    // Where the range is tiny against the zero-point the levels themselves round together, and near
+    // the top of float32's range (or beyond it: infinities, a NaN mean) borders and steps overflow:
     // everything again.
     const float range = mode == TQ_KEYS_UNIFORM ? 15.0f * amax : amax;
-    s_tol[d] = range >= fabsf(mu) * (1.0f / 512.0f) ? (fabsf(mu) + range) * 0x1p-19f : INFINITY;
+    const bool plain = range >= fabsf(mu) * (1.0f / 512.0f) && fabsf(mu) + range < 0x1p126f;
+    s_tol[d] = plain ? (fabsf(mu) + range) * 0x1p-19f : INFINITY;
   } else if (!F32 && tid < TQ_D + 64) {  // packed: a thread per channel pair
     const uint32_t* gm = (const uint32_t*)tab + (tid - TQ_D);
     uint32_t top[EK_K];
@@ -461,7 +463,9 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k) out[(8 * c + k) * (TQ_D / 2)] = (uint8_t)code[k];
-      if (m0 < tol0 || m1 < tol1)
+      // (not closer than the tolerance: a channel that is computed again as a whole has an infinite
+      // one, and its minima may be infinite too)
+      if (!(m0 > tol0) || !(m1 > tol1))
         redos[atomicAdd(&s_n_redo, 1)] = (unsigned short)(p | ((t0 / 8 + c) << 6));
     }
   }
@@ -471,19 +475,33 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   {
     // The reference's nearest level: the first minimum of the rounded distances.  An element
     // close to a border has one of the two levels beside it (the code found, or a neighbour);
-    // where the levels themselves round together all sixteen are tried.
+    // where the levels themselves round together all sixteen are tried.  Channels near or beyond
+    // the top of float32's range get the general encoder's two candidates of a bin, so that both
+    // give them the same codes.
     auto exact_code = [&](float v, float mu, float sc, float tol, int c) -> int {
       if (mode == TQ_KEYS_UNIFORM) {
         const float qv = rintf(__fdiv_rn(__fsub_rn(v, mu), sc));  // ties to even, like np.round
         return (int)fminf(fmaxf(qv, 0.0f), 15.0f);
       }
-      const bool all = isinf(tol);
-      const int l_lo = all ? 0 : max(c - 1, 0), l_hi = all ? 15 : min(c + 1, 15);
-      int best = l_lo;
-      float bd = INFINITY;
-      for (int l = l_lo; l <= l_hi; ++l) {
+      auto dist = [&](int l) -> float {
         const float sl = __fmul_rn(sc, s_grid[l]);
-        const float dv = fabsf(__fsub_rn(v, mode == TQ_KEYS_NF4 ? sl : __fadd_rn(mu, sl)));
+        return fabsf(__fsub_rn(v, mode == TQ_KEYS_NF4 ? sl : __fadd_rn(mu, sl)));
+      };
+      int l_lo = max(c - 1, 0), l_hi = min(c + 1, 15);
+      if (isinf(tol)) {
+        l_lo = 0;
+        l_hi = 15;
+        if (sc >= fabsf(mu) * (1.0f / 512.0f)) {
+          const int bin = min(max(__float2int_rd(fmaf(v - mu, 32.0f / sc, 32.0f)), 0), 63);
+          const float left = -1.0f + (float)bin * (1.0f / 32.0f) - 1.0e-4f;
+          for (int l = 0; l < 15; ++l) l_lo += (0.5f * (s_grid[l] + s_grid[l + 1]) < left) ? 1 : 0;
+          l_hi = min(l_lo + 1, 15);
+        }
+      }
+      int best = l_lo;
+      float bd = dist(l_lo);  // (a NaN stays: nothing is less)
+      for (int l = l_lo + 1; l <= l_hi; ++l) {
+        const float dv = dist(l);
         if (dv < bd) {
           bd = dv;
           best = l;
