@@ -148,3 +148,22 @@ def test_keys_at_and_beyond_the_top_of_the_range(dt, mode):
         idx, val = _outliers(x[blk * S:(blk + 1) * S], 5)
         assert np.array_equal(got["outlier_idx"], idx)
         assert np.array_equal(got["outlier_val"].view(np.uint16), val)
+
+
+@pytest.mark.parametrize("dt", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("mode", ["nf4_asym", "nf4", "uniform"])
+def test_channels_of_nan_have_the_general_encoder_s_extremes(dt, mode):
+    import torch
+
+    n = W + 2 * S
+    x = np.random.default_rng(4).standard_normal((n, H, 128)).astype(np.float32)
+    x[:, 0, 2] = np.nan
+    x[:, 1, 5] = np.nan
+    x[70, 1, 5] = -3.0                           # a single number
+    x[:64, 0, 9] = np.nan                        # the tokens of some threads
+    x[0, 0, 11] = np.nan                         # a first token
+    t = torch.from_numpy(x).to(getattr(torch, dt))
+    for got, want in zip(_blocks(t, mode, 0.02, dt)[:2], _blocks(t, mode, 0.036, dt)[:2], strict=True):
+        assert np.array_equal(got["key_indices"], want["key_indices"])
+        assert np.array_equal(got["nf4_scale"], want["nf4_scale"])
+        assert np.array_equal(got["nf4_mean"], want["nf4_mean"], equal_nan=True)

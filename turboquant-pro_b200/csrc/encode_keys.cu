@@ -255,7 +255,8 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
       *(float2*)&s_mn[seg * TQ_D + 2 * p] = mn;
       *(float2*)&s_mx[seg * TQ_D + 2 * p] = mx;
     } else {
-      uint32_t mn = ldw(t0), mx = mn, gm[GPT];
+      constexpr uint32_t PINF = BF ? 0x7F807F80u : 0x7C007C00u;
+      uint32_t mn = PINF, mx = PINF | 0x80008000u, gm[GPT];  // (not a first token: it may be NaN)
 #pragma unroll
       for (int j = 0; j < GPT; ++j) gm[j] = 0u;
 #pragma unroll 1
