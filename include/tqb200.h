@@ -332,11 +332,14 @@ int32_t tq_clear(tq_ctx* ctx, int32_t layer, int32_t seq, void* stream);
 
 /* Reads and clears the device status word.  Synchronises `stream`.
  *   bit 0 (1): an outlier pool overflowed and a block kept a truncated side-list;
- *   bit 1 (2): a bounded wait inside the tensor-core decode kernel ran out (a tile copy did
- *              not arrive within the limit), or one inside the tcgen05 value encoder.  The kernel then stops waiting and returns, so
- *              the device stays usable, but the `out` / `mlo` of that call is undefined:
- *              tq_decode itself has already returned TQ_OK (it does not synchronise), so a
- *              caller that wants the guarantee reads the status after the call. */
+ *   bit 1 (2): a bounded wait ran out and the kernel returned, so the device stays usable:
+ *              - in the tensor-core decode kernel (a tile copy did not arrive within the limit):
+ *                the `out` / `mlo` of that call is undefined;
+ *              - in an encoder, on tq_append: a block was stored that does not hold its tokens (the
+ *                key encoder for 256-token blocks stores an empty key block: keys of zero), so the
+ *                sequence has to be cleared and appended again.
+ * The calls themselves have already returned TQ_OK (they do not synchronise), so a caller that
+ * wants the guarantee reads the status after the call. */
 int32_t tq_status(tq_ctx* ctx, int32_t* flags, void* stream);
 
 /* Chooses, for the whole process, the kernel that rotates and quantises values (and, in
@@ -403,12 +406,13 @@ int32_t tq_set_kernel(tq_ctx* ctx, int32_t which);
  * kv_fused_pck.py:216-236); no direct counterpart. */
 int32_t tq_last_kernel(const tq_ctx* ctx);
 
-/* Test hook for the bounded waits of the tensor-core decode kernel (no counterpart in the
- * reference).  `wait_limit` > 0 replaces the number of probes a wait makes before it gives up
- * (0 restores the default, about half a second); `withhold_tile` >= 0 makes the first CTA of
- * later decodes never start the copy of that tile of its share, so that the wait for it runs
- * out and bit 1 of the status word is set (-1 switches this off).  Nothing faults and nothing
- * spins without bound; used by the tests of the error path. */
+/* Test hook for the bounded waits of the tensor-core decode kernel and of the key encoder for
+ * 256-token blocks (no counterpart in the reference).  `wait_limit` > 0 replaces the number of
+ * probes a wait makes before it gives up (0 restores the defaults, at most about half a second);
+ * `withhold_tile` >= 0 makes the first CTA of later decodes never start the copy of that tile of
+ * its share, and the first CTA of later appends that of the row of that number of its block, so
+ * that the wait for it runs out and bit 1 of the status word is set (-1 switches this off).
+ * Nothing faults and nothing spins without bound; used by the tests of the error path. */
 int32_t tq_debug_wait(tq_ctx* ctx, int32_t wait_limit, int32_t withhold_tile);
 
 /* Pipeline trace of the tensor-core decode kernel (debugging aid, no counterpart in the

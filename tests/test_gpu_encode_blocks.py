@@ -167,3 +167,42 @@ def test_channels_of_nan_have_the_general_encoder_s_extremes(dt, mode):
         assert np.array_equal(got["key_indices"], want["key_indices"])
         assert np.array_equal(got["nf4_scale"], want["nf4_scale"])
         assert np.array_equal(got["nf4_mean"], want["nf4_mean"], equal_nan=True)
+
+
+@pytest.mark.parametrize("dt", ["float16", "float32"])
+def test_a_block_that_does_not_arrive_is_stored_empty(dt):
+    """The test hook withholds one row of the first block; the wait for it runs out, the status word
+    says so, and the cache holds zeros in that block's place."""
+    import torch
+
+    from turboquant_pro_b200 import KVContext
+
+    n = W + 2 * S
+    x = np.random.default_rng(6).standard_normal((n, H, 128)).astype(np.float32)
+    kt = torch.from_numpy(x).to(getattr(torch, dt))[None].cuda()
+    good, ctx = (KVContext(n_layers=1, n_seqs=1, n_kv_heads=H, n_q_heads=H, value_bits=3,
+                           hot_window=W, max_tokens_per_seq=n, kv_dtype=dt, seed=5)
+                 for _ in range(2))
+    good.append(0, kt, kt)
+    want_k, want_v = good.dequant(0, 0, 0, n)
+    ctx._regions["pages"].fill_(0x5A)  # what an earlier user of the pages left there
+    ctx.debug_wait(wait_limit=256, withhold_tile=17)
+    ctx.append(0, kt, kt)
+    assert ctx.status() == 2 and ctx.status() == 0
+    ctx.debug_wait()
+    k, v = ctx.dequant(0, 0, 0, n)
+    assert not k[0, :S].any()
+    assert torch.equal(k[0, S:], want_k[0, S:]) and torch.equal(k[1], want_k[1])
+    assert torch.equal(v, want_v)
+    blk = ctx.export_block(0, 0, 0)
+    assert (blk["outlier_idx"] >= S * 128).all() and not blk["nf4_scale"][0, 0].any()
+    q = torch.randn((1, H, 128), device="cuda")
+    s = torch.einsum("hd,htd->ht", q[0].double(), k.double()) / 128 ** 0.5
+    want = torch.einsum("ht,htd->hd", s.softmax(-1), v.double())
+    for kernel in ("auto", "general"):
+        ctx.set_kernel(kernel)
+        # (the scores' outlier corrections are stored in fp16: about 3e-4 of a score of one)
+        assert ((ctx.decode(0, q)[0] - want).norm() / want.norm()).item() < 5e-3
+    ctx.clear(0, 0)
+    ctx.append(0, kt, kt)
+    assert ctx.status() == 0 and torch.equal(ctx.dequant(0, 0, 0, n)[0], want_k)

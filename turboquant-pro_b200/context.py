@@ -273,12 +273,12 @@ class KVContext:
         return out
 
     def raise_on_timeout(self) -> int:
-        """Reads the status word (synchronises); raises if a bounded wait of a decode kernel ran
-        out since the last read, else returns the other flags."""
+        """Reads the status word (synchronises); raises if a bounded wait of a kernel ran out since
+        the last read, else returns the other flags."""
         flags = self.status()
         if flags & 2:
-            raise _lib.TqError(-3, "a bounded wait inside the decode kernel ran out; the "
-                                   "output of that call is undefined")
+            raise _lib.TqError(-3, "a bounded wait inside a kernel ran out: the output of that decode "
+                                   "is undefined, or that append stored a block without its tokens")
         return flags
 
     def decode_static_scratch(self, layer: int, q, out=None):
@@ -668,8 +668,9 @@ class KVContext:
             check(self._lib.tq_clear(self._h, layer, seq, self._stream()))
 
     def status(self) -> int:
-        """Device status flags (bit 0: an outlier pool overflowed; bit 1: a bounded wait of the
-        tensor-core decode kernel ran out and that call's output is undefined); clears them."""
+        """Device status flags (bit 0: an outlier pool overflowed; bit 1: a bounded wait ran out:
+        in the tensor-core decode kernel, and that call's output is undefined, or in an append,
+        which then stored a block without its tokens: clear the sequence); clears them."""
         f = C.c_int32()
         with self._here():
             check(self._lib.tq_status(self._h, C.byref(f), self._stream()))
@@ -724,8 +725,9 @@ class KVContext:
         return {0: "none", 1: "tensor-core", 2: "general"}[int(self._lib.tq_last_kernel(self._h))]
 
     def debug_wait(self, wait_limit: int = 0, withhold_tile: int = -1) -> None:
-        """Test hook of the decode kernel's bounded waits: a shorter probe limit and a tile of
-        the first CTA whose copy is never started (see ``tq_debug_wait``)."""
+        """Test hook of the bounded waits of the decode kernel and the key encoder: a shorter probe
+        limit and a tile (a row) of the first CTA whose copy is never started (see
+        ``tq_debug_wait``)."""
         check(self._lib.tq_debug_wait(self._h, int(wait_limit), int(withhold_tile)))
 
     def trace(self, on: bool, read: bool = False):

@@ -1648,6 +1648,8 @@ int tq_launch_encode(tq_ctx* ctx, int layer, int seq_begin, int seq_count, const
   a.n_tokens = n_tokens;
   a.max_new_blocks = max_new_blocks;
   a.polar_keys_pass = 0;
+  a.wait_limit = ctx->wait_limit;
+  a.withhold_row = ctx->withhold_tile;
   a.seq_stride = seq_stride;
   a.tok_stride = tok_stride;
   a.head_stride = head_stride;

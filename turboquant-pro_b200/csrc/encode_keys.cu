@@ -28,6 +28,7 @@ constexpr int EK_S = 256;       // tokens per block
 constexpr int EK_K = 8;         // most outliers per channel and block
 constexpr int EK_BINS = 32;
 constexpr int EK_GROUPS = 32;   // groups of eight tokens per block
+constexpr int EK_WAIT = 1 << 16;  // probes for the block's copies before the CTA gives up
 constexpr float EK_MAGIC = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
 
 template <int DT>
@@ -168,7 +169,8 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     }
     __syncthreads();
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ek_smem);
-    if (tid < EK_S)
+    const bool held = tid == a.withhold_row && blockIdx.x + blockIdx.y + blockIdx.z == 0;  // test hook
+    if (tid < EK_S && !held)
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
               dst + tid * ROW_BYTES),
@@ -190,19 +192,36 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   if (tid < 16) s_grid[tid] = a.tables->grid[tid];
   if (tid == 0) s_n_redo = 0;
   for (int i = tid; i < EK_S * 4; i += THREADS) mask[i] = 0u;
-  if (aligned) {  // (bounded; a copy that never lands sets the status word)
+  auto landed = [&]() -> bool {  // bounded
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+    const int limit = a.wait_limit > 0 ? a.wait_limit : EK_WAIT;
     unsigned done = 0;
-    for (int i = 0; i < (1 << 16) && !done; ++i)
+    for (int i = 0; i < limit && !done; ++i)
       asm volatile(
           "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
           "selp.u32 %0, 1, 0, p;\n\t}\n"
           : "=r"(done)
           : "r"(bar)
           : "memory");
-    if (!done) atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+    return done != 0;
+  };
+  if (__syncthreads_or(aligned && !landed())) {
+    // A copy did not arrive: nothing is encoded from rows that are not there.  The status word says
+    // so, the page becomes an empty one (scales, zero-points and corrections of zero), and the
+    // copies still on their way get another bounded wait before the CTA gives up its shared memory.
+    if (tid == 0) {
+      atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+      a.page_meta[unit_index(g, a.layer, seq, head) * g.max_blocks + blk] = {0u, 0u};
+      landed();
+    }
+    auto zero = [&](int from, int to) {  // (multiples of 16, as all parts of a page are)
+      for (int i = from + 16 * tid; i < to; i += 16 * THREADS) *(uint4*)(page + i) = make_uint4(0, 0, 0, 0);
+    };
+    zero(0, g.k_bytes);
+    zero(g.scale_off, g.page_bytes);
+    __syncthreads();
+    return;
   }
-  __syncthreads();
 
   // ---- pass 1: sum in token order, extremes, group maxima -------------------------------------
   // The sum is a chain over all tokens: a segment's threads take it over from the segment before
