@@ -75,3 +75,33 @@ def test_batched_export_of_polarquant_keys():
         for name, x in want.items():
             same = x.tobytes() == got[name].tobytes() if isinstance(x, np.ndarray) else x == got[name]
             assert same, name
+
+
+def test_imports_of_two_geometries_from_two_threads():
+    """The kernel's shared-memory limit is the device's, not the context's: imports of a small page
+    beside imports of the largest one."""
+    import threading
+
+    import torch
+
+    from turboquant_pro_b200 import KVContext
+
+    jobs, errors = [], []
+    for w, vb, n in ((512, 4, 1100), (37, 3, 200)):
+        src, _, _, kw = _context(torch, w, vb, "float16", n, frac=0.0)
+        blks = [src.export_block(1, 1, b) for b in range(src.cold_blocks(n))]
+        jobs.append((KVContext(**kw), blks))
+
+    def work(ctx, blks):
+        try:
+            for _ in range(1500):
+                ctx._import_blocks(1, 1, 0, blks[:1])
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors

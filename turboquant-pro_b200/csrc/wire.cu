@@ -17,6 +17,11 @@
 namespace {
 
 constexpr int WIRE_THREADS = 256;
+// Dynamic shared memory a launch may ask for: the largest page (256 tokens, 4-bit values: 38 KB) and
+// its value codes as a bit stream (16 KB).  The limit belongs to the kernel on a device, not to a
+// context: it is set once, to the same value whoever comes first, so that no thread's small geometry
+// can take it away between another's look and launch.
+constexpr int WIRE_SMEM = 64 * 1024;
 
 struct WireParts {
   int64_t key, scale, mean, val, norm, bytes;  // offsets of a block's parts, bytes of a block
@@ -316,8 +321,12 @@ bool range_ok(const tq_ctx* ctx, int layer, int seq) {
 }
 
 template <class K>
-int allow_smem(K kernel, int bytes) {
-  TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+int allow_smem(K kernel, int bytes, int device, bool (&set)[64]) {
+  TQ_REQUIRE(bytes <= WIRE_SMEM, TQ_ERR_UNSUPPORTED, "a page larger than the wire kernels take");
+  if (device >= 64 || !set[device]) {
+    TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WIRE_SMEM));
+    if (device < 64) set[device] = true;
+  }
   return TQ_OK;
 }
 
@@ -375,7 +384,8 @@ int32_t tq_export_blocks(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t block,
   a.out_idx = outlier_idx;
   a.out_val = outlier_val;
   a.n_out = n_outliers;
-  const int rc = allow_smem(export_kernel, g.hdr_off);
+  static bool attr_set[64] = {};  // per device
+  const int rc = allow_smem(export_kernel, g.hdr_off, ctx->device, attr_set);
   if (rc != TQ_OK) return rc;
   export_kernel<<<dim3(g.n_kv_heads, n_blocks), WIRE_THREADS, g.hdr_off, (cudaStream_t)stream>>>(a);
   TQ_CUDA(cudaGetLastError());
@@ -405,10 +415,12 @@ int32_t tq_import_blocks(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t block,
   a.first = first;
   a.short_flag = short_flag;
   const int smem = g.page_bytes + g.block_tokens * 16 * g.value_bits;
-  const int rc = allow_smem(import_kernel, smem);
+  static bool attr_set[64] = {};  // per device
+  const int rc = allow_smem(import_kernel, smem, ctx->device, attr_set);
   if (rc != TQ_OK) return rc;
   TQ_CUDA(cudaMemsetAsync(short_flag, 0, 4, st));
   import_kernel<<<dim3(g.n_kv_heads, n_blocks), WIRE_THREADS, smem, st>>>(a);
+  TQ_CUDA(cudaGetLastError());  // (no page written: the cursors stay)
   import_cursor_kernel<<<(g.n_kv_heads + 127) / 128, 128, 0, st>>>(a);
   TQ_CUDA(cudaGetLastError());
   int32_t lacking = 0;
