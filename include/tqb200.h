@@ -251,10 +251,11 @@ int32_t tq_dequant_range(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t start,
 
 /* The first n_tokens tokens of one sequence, dequantised as by tq_dequant_range, rounded to `dtype`
  * (TQ_F32, TQ_F16 or TQ_BF16) and written to the rows of an engine's paged tensors: token t goes to
- * row t % page_tokens of page page_ids[t / page_tokens] (device array; the caller vouches that every
- * id names a page).  Strides in elements; a row's channels are contiguous. */
+ * row t % page_tokens of page page_ids[t / page_tokens] (device array).  The tokens of an id outside
+ * [0, n_pages) are not written, and bit 2 of the status word is set.  Strides in elements; a row's
+ * channels are contiguous. */
 int32_t tq_dequant_paged(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t n_tokens, void* k_pages,
-                         void* v_pages, int32_t dtype, const int64_t* page_ids,
+                         void* v_pages, int32_t dtype, const int64_t* page_ids, int64_t n_pages,
                          int32_t page_tokens, int64_t page_stride, int64_t row_stride,
                          int64_t head_stride, void* stream);
 
@@ -338,6 +339,7 @@ int32_t tq_clear(tq_ctx* ctx, int32_t layer, int32_t seq, void* stream);
  *              - in an encoder, on tq_append: a block was stored that does not hold its tokens (the
  *                key encoder for 256-token blocks stores an empty key block: keys of zero), so the
  *                sequence has to be cleared and appended again.
+ *   bit 2 (4): tq_dequant_paged met a page id outside the tensor and left its tokens out.
  * The calls themselves have already returned TQ_OK (they do not synchronise), so a caller that
  * wants the guarantee reads the status after the call. */
 int32_t tq_status(tq_ctx* ctx, int32_t* flags, void* stream);

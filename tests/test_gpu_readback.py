@@ -100,3 +100,31 @@ def test_restore_into_pages_equals_the_dense_read_back(dt, layout):
     with pytest.raises(ValueError):
         store.load_into_paged("r", 1, kv, table[:-(-n // bs) - 1])
     assert store.load_into_paged("r", 0, kv, table) == 0
+
+
+@pytest.mark.parametrize("mode", ["nf4_asym", "polar"])
+def test_tokens_of_a_page_outside_the_tensor_are_left_out(mode):
+    import torch
+
+    from turboquant_pro_b200 import KVContext
+    from turboquant_pro_b200.synth import make_kv
+
+    n, bs, pages = 777, 7, 120
+    polar = mode == "polar"
+    ctx = KVContext(n_kv_heads=H, value_bits=3, key_bits=3 if polar else 4, key_mode=mode,
+                    outlier_frac=0.0 if polar else 0.02, max_tokens_per_seq=n, kv_dtype="float16", seed=4)
+    k, v = (torch.from_numpy(x)[None].cuda() for x in make_kv(8, H, n, dtype=np.float16))
+    ctx.append(0, k, v)
+    kv = torch.zeros((2, pages, bs, H, 128), dtype=torch.float16, device="cuda")
+    ids = torch.randperm(pages, generator=torch.Generator().manual_seed(1))[:-(-n // bs)]
+    ctx.dequant_into_pages(0, 0, n, kv[0], kv[1], ids.cuda())
+    assert ctx.status() == 0
+    want = kv.clone()
+    bad = ids.clone()
+    for at, i in ((2, pages), (5, -1), (40, -(1 << 40)), (len(ids) - 1, 1 << 40)):
+        want[:, ids[at]] = 0.0  # (cold pages and one of the window)
+        bad[at] = i
+    kv.zero_()
+    ctx.dequant_into_pages(0, 0, n, kv[0], kv[1], bad.cuda())
+    assert torch.equal(kv, want)
+    assert ctx.status() == 4 and ctx.status() == 0

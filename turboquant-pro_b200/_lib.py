@@ -92,8 +92,8 @@ SIGNATURES = {
     "tq_dequant_range": (C.c_int32, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                      C.c_void_p, C.c_void_p, C.c_void_p]),
     "tq_dequant_paged": (C.c_int32, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,
-                                     C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int64,
-                                     C.c_int64, C.c_int64, C.c_void_p]),
+                                     C.c_void_p, C.c_int32, C.c_void_p, C.c_int64, C.c_int32,
+                                     C.c_int64, C.c_int64, C.c_int64, C.c_void_p]),
     "tq_export_block": (C.c_int32, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,
                                     C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32,
                                     C.POINTER(C.c_int32), C.c_void_p, C.c_void_p, C.c_void_p]),

@@ -192,8 +192,10 @@ class DeviceBlockStore:
                 and tuple(kv_layer.shape[3:]) == (g.n_kv_heads, g.head_dim) \
                 and kv_layer.dtype in (torch.float32, torch.float16, torch.bfloat16) \
                 and type(kv_layer) is torch.Tensor and not kv_layer.requires_grad:
-            # straight from the codes to the engine's rows; the lookup refuses ids outside the
-            # tensor (and counts negative ones from its end) as indexing the pages would
+            # straight from the codes to the engine's rows; the lookup counts negative ids from the
+            # tensor's end and stops at ids outside it as indexing the pages would (on CUDA a
+            # device-side assertion, after which the process has to start again; the kernel itself
+            # leaves such ids out)
             pages = torch.arange(kv_layer.shape[1], device=kv_layer.device)[ids[:-(-n // bs)]]
             ctx.dequant_into_pages(layer, slot, n, kv_layer[0], kv_layer[1], pages)
             if not kv_layer.is_inference():  # (an inference tensor keeps no version)

@@ -363,8 +363,8 @@ class KVContext:
         """Writes the first ``n_tokens`` dequantised tokens into an engine's pages: token ``t`` to
         row ``t % page_tokens`` of page ``ids[t // page_tokens]`` of ``k_pages`` / ``v_pages``
         ``[n_pages, page_tokens, n_kv_heads, D]`` (one element type and layout, channels
-        contiguous; float32, float16 or bfloat16).  ``ids`` is an int64 CUDA tensor whose entries
-        the caller has checked."""
+        contiguous; float32, float16 or bfloat16).  ``ids`` is an int64 CUDA tensor; the tokens of
+        an entry outside ``[0, n_pages)`` are left out and :meth:`status` reports bit 2."""
         g = self.geom
         if k_pages.shape != v_pages.shape or k_pages.stride() != v_pages.stride() \
                 or k_pages.dtype != v_pages.dtype or k_pages.device != self.device \
@@ -378,8 +378,8 @@ class KVContext:
         with self._here():
             check(self._lib.tq_dequant_paged(
                 self._h, layer, seq, n_tokens, k_pages.data_ptr(), v_pages.data_ptr(),
-                _dtype_code(k_pages.dtype), ids.data_ptr(), k_pages.shape[1], k_pages.stride(0),
-                k_pages.stride(1), k_pages.stride(2), self._stream()))
+                _dtype_code(k_pages.dtype), ids.data_ptr(), k_pages.shape[0], k_pages.shape[1],
+                k_pages.stride(0), k_pages.stride(1), k_pages.stride(2), self._stream()))
 
     def export_block(self, layer: int, seq: int, block: int) -> dict:
         """Cold block ``block`` in the reference's container layout (host numpy arrays):
@@ -670,7 +670,8 @@ class KVContext:
     def status(self) -> int:
         """Device status flags (bit 0: an outlier pool overflowed; bit 1: a bounded wait ran out:
         in the tensor-core decode kernel, and that call's output is undefined, or in an append,
-        which then stored a block without its tokens: clear the sequence); clears them."""
+        which then stored a block without its tokens: clear the sequence; bit 2:
+        :meth:`dequant_into_pages` met a page outside the tensor); clears them."""
         f = C.c_int32()
         with self._here():
             check(self._lib.tq_status(self._h, C.byref(f), self._stream()))

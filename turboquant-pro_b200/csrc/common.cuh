@@ -38,6 +38,7 @@ constexpr int TQ_PAGE_SPILLED = 1;  // header flag: use the pool's list, not the
 // stored a block that does not hold its tokens)
 constexpr int TQ_STATUS_POOL_OVERFLOW = 1;
 constexpr int TQ_STATUS_WAIT_TIMEOUT = 2;
+constexpr int TQ_STATUS_BAD_PAGE = 4;  // a page id outside the engine's tensor; its tokens were left out
 
 // which decode kernel served the most recent call (tq_last_kernel)
 constexpr int TQ_KERNEL_NONE = 0, TQ_KERNEL_TENSOR_CORE = 1, TQ_KERNEL_GENERAL = 2;
@@ -253,8 +254,8 @@ int tq_launch_lse_combine(const float* mlo, int n_parts, int n_rows, int head_di
 int tq_launch_dequant(tq_ctx* ctx, int layer, int seq, int start, int end, float* k_out,
                       float* v_out, cudaStream_t st);
 int tq_launch_dequant_paged(tq_ctx* ctx, int layer, int seq, int n_tokens, void* k_pages,
-                            void* v_pages, int dtype, const int64_t* page_ids, int page_tokens,
-                            int64_t page_stride, int64_t row_stride, int64_t head_stride,
-                            cudaStream_t st);
+                            void* v_pages, int dtype, const int64_t* page_ids, int64_t n_pages,
+                            int page_tokens, int64_t page_stride, int64_t row_stride,
+                            int64_t head_stride, cudaStream_t st);
 size_t tq_mma_scratch_bytes(const tq_geom& g, size_t units);
 int tq_launch_clear(tq_ctx* ctx, int layer, int seq_begin, int seq_count, cudaStream_t st);

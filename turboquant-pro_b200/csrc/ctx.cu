@@ -405,7 +405,7 @@ int32_t tq_dequant_range(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t start,
 }
 
 int32_t tq_dequant_paged(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t n_tokens, void* k_pages,
-                         void* v_pages, int32_t dtype, const int64_t* page_ids,
+                         void* v_pages, int32_t dtype, const int64_t* page_ids, int64_t n_pages,
                          int32_t page_tokens, int64_t page_stride, int64_t row_stride,
                          int64_t head_stride, void* stream) {
   TQ_REQUIRE(good_ctx(ctx, layer), TQ_ERR_INVALID, "bad context or layer");
@@ -416,8 +416,9 @@ int32_t tq_dequant_paged(tq_ctx* ctx, int32_t layer, int32_t seq, int32_t n_toke
   TQ_REQUIRE(page_tokens >= 1, TQ_ERR_INVALID, "page_tokens must be positive");
   if (n_tokens == 0 || (k_pages == nullptr && v_pages == nullptr)) return TQ_OK;
   TQ_REQUIRE(page_ids != nullptr, TQ_ERR_INVALID, "page_ids must be a device pointer");
+  TQ_REQUIRE(n_pages >= 0, TQ_ERR_INVALID, "n_pages must not be negative");
   TQ_CUDA(cudaSetDevice(ctx->device));
-  return tq_launch_dequant_paged(ctx, layer, seq, n_tokens, k_pages, v_pages, dtype, page_ids,
+  return tq_launch_dequant_paged(ctx, layer, seq, n_tokens, k_pages, v_pages, dtype, page_ids, n_pages,
                                  page_tokens, page_stride, row_stride, head_stride,
                                  (cudaStream_t)stream);
 }

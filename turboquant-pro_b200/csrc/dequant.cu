@@ -46,8 +46,11 @@ struct DequantArgs {
   void* k_out;
   void* v_out;
   // row of (position, head): dense, head_stride * head + row_stride * (position - start); paged,
-  // ids[position / page_tokens] * page_stride + (position % page_tokens) * row_stride + head_stride * head
+  // ids[position / page_tokens] * page_stride + (position % page_tokens) * row_stride + head_stride * head,
+  // nothing (and a status bit) where the id is outside [0, pages)
   const int64_t* ids;
+  int64_t pages_out;
+  int32_t* status;
   int page_tokens;
   int64_t page_stride, row_stride, head_stride;
   float one;    // 1.0f (see dq_add2)
@@ -102,14 +105,17 @@ TQ_DEV void store4(typename Elem<OT>::type* p, float a, float b, float c, float 
   }
 }
 
-template <int OT>
+// (null: the row has no place)
+template <int OT, bool PAGED>
 TQ_DEV typename Elem<OT>::type* out_row(const DequantArgs& a, void* base, int pos, int head) {
   int64_t o;
-  if (a.ids == nullptr)
+  if constexpr (PAGED) {
+    const int64_t id = a.ids[pos / a.page_tokens];
+    if ((uint64_t)id >= (uint64_t)a.pages_out) return nullptr;
+    o = id * a.page_stride + (pos % a.page_tokens) * a.row_stride + head * a.head_stride;
+  } else {
     o = (int64_t)head * a.head_stride + (int64_t)(pos - a.start) * a.row_stride;
-  else
-    o = a.ids[pos / a.page_tokens] * a.page_stride + (pos % a.page_tokens) * a.row_stride +
-        head * a.head_stride;
+  }
   return (typename Elem<OT>::type*)base + o;
 }
 
@@ -134,7 +140,7 @@ TQ_DEV void ld4_any(const void* p, size_t i, int dt, float (&x)[4]) {
   }
 }
 
-template <int OT>
+template <int OT, bool PAGED>
 __global__ void __launch_bounds__(DQ_THREADS, 2) dequant_kernel(DequantArgs a) {
   const tq_geom& g = a.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -157,6 +163,13 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) dequant_kernel(DequantArgs a) {
                    : "memory");
   }
   __syncthreads();
+  // (a page without a place is reported once, at the end: no atomic among the loads and stores)
+  bool missed = false;
+  auto has_place = [&](const void* row) -> bool {
+    if (!PAGED || row != nullptr) return true;
+    missed = true;
+    return false;
+  };
 
   auto key_job = [&](int job) {
     const int kt = job % a.k_tiles, pg = job / a.k_tiles % a.n_pages,
@@ -177,23 +190,34 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) dequant_kernel(DequantArgs a) {
     }
     const float4 sc = *(const float4*)(page + g.scale_off + 16 * lane);
     const float4 mu = *(const float4*)(page + g.mean_off + 16 * lane);
-#pragma unroll 4
-    for (int t = lo + warp; t < hi; t += DQ_THREADS / 32) {
-      const uint32_t w = *(const uint16_t*)(page + t * (TQ_D / 2) + 2 * lane);
-      // symmetric NF4 stores mean 0, uniform keys are fl(fl(code * scale) + zero): one form
-      store4<OT>(out_row<OT>(a, a.k_out, blk * S + t, head) + 4 * lane,
-                 __fadd_rn(__fmul_rn(sc.x, grid_s[w & 15]), mu.x),
-                 __fadd_rn(__fmul_rn(sc.y, grid_s[(w >> 4) & 15]), mu.y),
-                 __fadd_rn(__fmul_rn(sc.z, grid_s[(w >> 8) & 15]), mu.z),
-                 __fadd_rn(__fmul_rn(sc.w, grid_s[w >> 12]), mu.w), a.aligned);
+    constexpr int WARPS = DQ_THREADS / 32;
+    for (int t4 = lo + warp; t4 < hi; t4 += 4 * WARPS) {  // four rows: their loads, then their stores
+      typename Elem<OT>::type* row[4];
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = min(t4 + i * WARPS, hi - 1);
+        row[i] = out_row<OT, PAGED>(a, a.k_out, blk * S + t, head);
+        w[i] = *(const uint16_t*)(page + t * (TQ_D / 2) + 2 * lane);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        // symmetric NF4 stores mean 0, uniform keys are fl(fl(code * scale) + zero): one form
+        if (t4 + i * WARPS < hi && has_place(row[i]))
+          store4<OT>(row[i] + 4 * lane,
+                     __fadd_rn(__fmul_rn(sc.x, grid_s[w[i] & 15]), mu.x),
+                     __fadd_rn(__fmul_rn(sc.y, grid_s[(w[i] >> 4) & 15]), mu.y),
+                     __fadd_rn(__fmul_rn(sc.z, grid_s[(w[i] >> 8) & 15]), mu.z),
+                     __fadd_rn(__fmul_rn(sc.w, grid_s[w[i] >> 12]), mu.w), a.aligned);
+      }
     }
     if (pm.cnt == 0) return;
     __syncthreads();  // the rows are written; the outliers go over them
     auto put = [&](uint32_t w, uint32_t e) {
       const int col = (w >> 16) & 255, t = (int)(w >> 24);
       if (t < lo || t >= hi) return;
-      out_row<OT>(a, a.k_out, blk * S + t, head)[col] =
-          to_out<OT>(__half2float(__ushort_as_half(a.pool_val[slab + e])));
+      auto* row = out_row<OT, PAGED>(a, a.k_out, blk * S + t, head);
+      if (has_place(row)) row[col] = to_out<OT>(__half2float(__ushort_as_half(a.pool_val[slab + e])));
     };
 #pragma unroll
     for (int i = 0; i < DQ_PRE; ++i) {
@@ -213,14 +237,14 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) dequant_kernel(DequantArgs a) {
     for (int pos = p0 + warp; pos < min(p0 + DQ_HT, a.end); pos += DQ_THREADS / 32) {
       const size_t i = ring + (size_t)(pos % g.hot_cap) * TQ_D + 4 * lane;
       float x[4];
-      if (a.k_out) {
-        ld4_any(a.hot_k, i, g.kv_dtype, x);
-        store4<OT>(out_row<OT>(a, a.k_out, pos, head) + 4 * lane, x[0], x[1], x[2], x[3], a.aligned);
-      }
-      if (a.v_out) {
-        ld4_any(a.hot_v, i, g.kv_dtype, x);
-        store4<OT>(out_row<OT>(a, a.v_out, pos, head) + 4 * lane, x[0], x[1], x[2], x[3], a.aligned);
-      }
+      auto move = [&](const void* ring_of, void* to) {
+        if (to == nullptr) return;
+        auto* row = out_row<OT, PAGED>(a, to, pos, head);
+        ld4_any(ring_of, i, g.kv_dtype, x);
+        if (has_place(row)) store4<OT>(row + 4 * lane, x[0], x[1], x[2], x[3], a.aligned);
+      };
+      move(a.hot_k, a.k_out);
+      move(a.hot_v, a.v_out);
     }
   };
 
@@ -313,9 +337,11 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) dequant_kernel(DequantArgs a) {
           x[2 * j] = __fmul_rn(x[2 * j], nrm);
           x[2 * j + 1] = __fmul_rn(x[2 * j + 1], nrm);
         }
-        auto* row = out_row<OT>(a, polar ? a.k_out : a.v_out, blk * S + tt, head);
-        store4<OT>(row + 4 * tx, x[0], x[1], x[2], x[3], a.aligned);
-        store4<OT>(row + 64 + 4 * tx, x[4], x[5], x[6], x[7], a.aligned);
+        auto* row = out_row<OT, PAGED>(a, polar ? a.k_out : a.v_out, blk * S + tt, head);
+        if (has_place(row)) {
+          store4<OT>(row + 4 * tx, x[0], x[1], x[2], x[3], a.aligned);
+          store4<OT>(row + 64 + 4 * tx, x[4], x[5], x[6], x[7], a.aligned);
+        }
       }
     }
     __syncthreads();  // the expanded codes make room for the next job's
@@ -333,13 +359,14 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) dequant_kernel(DequantArgs a) {
       for (int j = first; j < nv_all; j += step) value_job(j);
     }
   }
+  if (missed) atomicOr(a.status, TQ_STATUS_BAD_PAGE);
 }
 
-template <int OT>
+template <int OT, bool PAGED>
 int launch_t(const DequantArgs& a, int device, cudaStream_t st) {
   static bool attr_set[64] = {};  // per device: the attribute belongs to the device's context
   if (device >= 64 || !attr_set[device]) {
-    TQ_CUDA(cudaFuncSetAttribute(dequant_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TQ_CUDA(cudaFuncSetAttribute(dequant_kernel<OT, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  DQ_SMEM));
     if (device < 64) attr_set[device] = true;
   }
@@ -347,7 +374,7 @@ int launch_t(const DequantArgs& a, int device, cudaStream_t st) {
   cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
   // one wave of resident CTAs: Pi is fetched once per CTA
   const int jobs = std::max(a.n_v + a.n_polar, a.n_k + a.n_h);
-  dequant_kernel<OT><<<std::min(jobs, 2 * sm_count), DQ_THREADS, DQ_SMEM, st>>>(a);
+  dequant_kernel<OT, PAGED><<<std::min(jobs, 2 * sm_count), DQ_THREADS, DQ_SMEM, st>>>(a);
   TQ_CUDA(cudaGetLastError());
   return TQ_OK;
 }
@@ -364,6 +391,7 @@ int launch(tq_ctx* ctx, DequantArgs& a, int layer, int seq, int start, int end, 
   a.pool_val = (const uint16_t*)ctx->b.pool_val;
   a.page_meta = (const PageMeta*)ctx->b.page_meta;
   a.tables = (const Tables*)ctx->b.tables;
+  a.status = (int32_t*)((uint8_t*)ctx->b.state + state_status_off(g));
   a.layer = layer;
   a.seq = seq;
   a.start = start;
@@ -386,10 +414,11 @@ int launch(tq_ctx* ctx, DequantArgs& a, int layer, int seq, int start, int end, 
   a.n_polar = a.k_out != nullptr && polar ? g.n_kv_heads * a.n_pages * a.v_tiles : 0;
   a.n_k = a.k_out != nullptr && !polar ? g.n_kv_heads * a.n_pages * a.k_tiles : 0;
   a.n_h = end > hbeg ? g.n_kv_heads * ((end - hbeg + DQ_HT - 1) / DQ_HT) : 0;
+  if (a.ids == nullptr) return launch_t<TQ_F32, false>(a, ctx->device, st);
   switch (dtype) {
-    case TQ_F32: return launch_t<TQ_F32>(a, ctx->device, st);
-    case TQ_F16: return launch_t<TQ_F16>(a, ctx->device, st);
-    default: return launch_t<TQ_BF16>(a, ctx->device, st);
+    case TQ_F32: return launch_t<TQ_F32, true>(a, ctx->device, st);
+    case TQ_F16: return launch_t<TQ_F16, true>(a, ctx->device, st);
+    default: return launch_t<TQ_BF16, true>(a, ctx->device, st);
   }
 }
 
@@ -406,13 +435,14 @@ int tq_launch_dequant(tq_ctx* ctx, int layer, int seq, int start, int end, float
 }
 
 int tq_launch_dequant_paged(tq_ctx* ctx, int layer, int seq, int n_tokens, void* k_pages,
-                            void* v_pages, int dtype, const int64_t* page_ids, int page_tokens,
-                            int64_t page_stride, int64_t row_stride, int64_t head_stride,
-                            cudaStream_t st) {
+                            void* v_pages, int dtype, const int64_t* page_ids, int64_t n_pages,
+                            int page_tokens, int64_t page_stride, int64_t row_stride,
+                            int64_t head_stride, cudaStream_t st) {
   DequantArgs a = {};
   a.k_out = k_pages;
   a.v_out = v_pages;
   a.ids = page_ids;
+  a.pages_out = n_pages;
   a.page_tokens = page_tokens;
   a.page_stride = page_stride;
   a.row_stride = row_stride;
