@@ -122,3 +122,25 @@ def test_facade_refuses_cpu():
     if not torch.cuda.is_available():
         with pytest.raises(RuntimeError, match="no CPU fallback"):
             TurboQuantKVCache.robust(n_heads=2)
+
+
+def test_stream_of_a_torch_without_the_raw_form(monkeypatch):
+    import types
+
+    import torch
+
+    from turboquant_pro_b200 import KVContext, context
+
+    ctx = object.__new__(KVContext)
+    ctx.device = torch.device("cuda", 3)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 1000 + index, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda device: types.SimpleNamespace(cuda_stream=2000 + device))
+    context._raw_stream.cache_clear()
+    try:
+        assert ctx._stream() == 1003
+        monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+        context._raw_stream.cache_clear()
+        assert ctx._stream() == 2003
+    finally:
+        context._raw_stream.cache_clear()

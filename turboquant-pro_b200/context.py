@@ -75,6 +75,15 @@ def _dtype_code(torch_dtype) -> int:
     return _dtype_codes()[torch_dtype]
 
 
+@functools.cache
+def _raw_stream():
+    """The function that gives a device's current stream as an integer: torch's private one, without
+    a Stream object, where this torch has it."""
+    cuda = _torch().cuda
+    return getattr(_torch()._C, "_cuda_getCurrentRawStream", None) or (
+        lambda index: cuda.current_stream(index).cuda_stream)
+
+
 def _torch_dtype(name):
     torch = _torch()
     if isinstance(name, torch.dtype):
@@ -165,7 +174,7 @@ class KVContext:
     # A decode step of a layer is some ten microseconds on the GPU, and so is a call made up of
     # torch's device guard and a Stream object: both are taken only as far as they are needed.
     def _stream(self):
-        return _torch()._C._cuda_getCurrentRawStream(self.device.index)
+        return _raw_stream()(self.device.index)
 
     def _here(self):
         """The device guard of a library call (the library selects its device itself; the guard
