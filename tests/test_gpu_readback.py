@@ -128,3 +128,41 @@ def test_tokens_of_a_page_outside_the_tensor_are_left_out(mode):
     ctx.dequant_into_pages(0, 0, n, kv[0], kv[1], bad.cuda())
     assert torch.equal(kv, want)
     assert ctx.status() == 4 and ctx.status() == 0
+
+
+def test_pages_that_are_more_than_their_storage():
+    """What indexing the pages refuses, negates or differentiates, the restore does too."""
+    import torch
+    from torch.autograd import forward_ad
+
+    from turboquant_pro_b200.connector import DeviceBlockStore
+    from turboquant_pro_b200.synth import make_kv
+
+    n, bs, pages = 600, 16, 60
+    store = DeviceBlockStore(1, H, max_requests=1, max_tokens=n, value_bits=3, dtype="float16", seed=4)
+    assert store.save("r", 0, *(torch.from_numpy(x).cuda() for x in make_kv(8, H, n, dtype=np.float16)))
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(1))[:-(-n // bs)].cuda()
+
+    def fresh():
+        return torch.zeros((2, pages, bs, H, 128), dtype=torch.float16, device="cuda")
+
+    want = fresh()
+    store.load_into_paged("r", 0, want, table)
+    assert want.any()
+    kv = torch._neg_view(fresh())
+    store.load_into_paged("r", 0, kv, table)
+    assert torch.equal(kv.resolve_neg(), want)
+    with torch.inference_mode():
+        kv = fresh()
+        store.load_into_paged("r", 0, kv, table)
+        assert torch.equal(kv, want)
+    with pytest.raises(RuntimeError, match="[Ii]nference"):
+        store.load_into_paged("r", 0, kv, table)
+    with forward_ad.dual_level():
+        kv = forward_ad.make_dual(fresh(), fresh() + 1.0)
+        store.load_into_paged("r", 0, kv, table)
+        primal, tangent = forward_ad.unpack_dual(kv)
+        assert torch.equal(primal, want) and not tangent[:, table[0]].any()
+    stack = torch.stack([fresh(), fresh()])
+    torch.func.vmap(lambda x: (store.load_into_paged("r", 0, x, table), x)[1])(stack)
+    assert torch.equal(stack[0], want) and torch.equal(stack[1], want)

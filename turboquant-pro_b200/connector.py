@@ -32,6 +32,24 @@ __all__ = ["DeviceBlockStore", "TurboQuantKVConnector", "KVConnectorRole", "regi
 _CONNECTOR_NAME = "TurboQuantConnectorB200"
 
 
+def _takes_raw_writes(t) -> bool:
+    """Whether a kernel that is handed ``t``'s address does what indexing ``t`` would: not where
+    torch has more to do than store elements (a gradient or a tangent to follow, a transform's
+    wrapper, a lazily negated view) or refuses the write (an inference tensor outside its mode)."""
+    import torch
+    from torch.autograd import forward_ad
+
+    if type(t) is not torch.Tensor or t.requires_grad or t.is_neg() \
+            or (t.is_inference() and not torch.is_inference_mode_enabled()) \
+            or forward_ad.unpack_dual(t).tangent is not None:
+        return False
+    try:
+        t.data_ptr()
+    except RuntimeError:  # (a wrapper without storage)
+        return False
+    return True
+
+
 class DeviceBlockStore:
     """Per-request compressed KV prefixes on one GPU.
 
@@ -191,7 +209,7 @@ class DeviceBlockStore:
         if kv_layer.dim() == 5 and kv_layer.device == ctx.device and kv_layer.stride(4) == 1 \
                 and tuple(kv_layer.shape[3:]) == (g.n_kv_heads, g.head_dim) \
                 and kv_layer.dtype in (torch.float32, torch.float16, torch.bfloat16) \
-                and type(kv_layer) is torch.Tensor and not kv_layer.requires_grad:
+                and _takes_raw_writes(kv_layer):
             # straight from the codes to the engine's rows; the lookup counts negative ids from the
             # tensor's end and stops at ids outside it as indexing the pages would (on CUDA a
             # device-side assertion, after which the process has to start again; the kernel itself
