@@ -398,7 +398,9 @@ int32_t tq_set_key_bias_means(tq_ctx* ctx, const float* means, void* stream);
 /* Selects the decode kernel: 0 = automatic (the tensor-core kernel where the geometry
  * allows: 256-token blocks, GQA group 1/2/4/8, any number of sequences; else the
  * general-shape kernel), 1 = always the general-shape float32 kernel.  Both compute the same
- * function; tests compare them; tq_last_kernel tells which one ran.  No counterpart in the
+ * function; tests compare them; tq_last_kernel tells which one ran.  (256-token blocks with more
+ * than four query heads per KV head have a float32 kernel of their own, a page at a time; it counts
+ * as the general-shape kernel and takes its place in both settings.)  No counterpart in the
  * reference. */
 int32_t tq_set_kernel(tq_ctx* ctx, int32_t which);
 

@@ -22,8 +22,10 @@ struct DecodeArgs {
   float scale;
 };
 
-// Query groups of five and more on 256-token blocks (per-channel keys) take the page kernel (at three
-// heads its sums came out a tenth further from 64 bits than the general kernel's; above, no further).
+// Query groups of five and more on 256-token blocks (per-channel keys) take the page kernel; its times
+// beside the general kernel's stand at its launch.  Distance from 64 bits over 40 to 12 000 tokens,
+// general kernel / page kernel: 1.18e-6 / 1.11e-6 at five heads, 1.13 / 1.06 at seven, 1.11 / 1.06 at
+// nine, 1.12 / 1.06 at sixteen.  (At three heads it came out a tenth further away: not taken.)
 TQ_HD bool tq_decode_pages_form(const tq_geom& g) {
   return g.block_tokens == 256 && g.key_mode != TQ_KEYS_POLAR && g.group > 4;
 }

@@ -3,9 +3,14 @@
 // general-shape kernel is asked for.  Same arithmetic as decode_generic.cu: float32 products and sums
 // throughout; the partials have its layout and go through its combine kernel.
 //
-// Bound by instruction issue.  decode_generic.cu looks every code up once per tile of four heads, a
+// Bound by latency, not by issue.  Counters of one launch (160 units of seven heads, 700 to 12 000
+// tokens, 422 us): 32 % of the issue slots, 2.5 warps per scheduler of which 0.4 can issue; of 7.9
+// cycles between two instructions of a warp 3.6 wait for global memory (codes, scales, norms and outlier
+// lists are fetched where they are used, between the page's four barriers); and the splits are uneven, the
+// busiest SM works 822 000 cycles, the average one 633 000.  168 registers hold it at three CTAs an
+// SM, with 40 bytes spilled.  decode_generic.cu looks every code up once per tile of four heads, a
 // 16-token group at a time; here a code is looked up once for eight heads and feeds packed
-// multiply-adds (two heads an instruction), about nine instructions per code and lane:
+// multiply-adds (two heads an instruction), sixteen instructions per code and lane in all:
 //   scores   a lane owns two tokens and walks their channels; the weights w = q * scale of a channel
 //            lie side by side for the heads, two broadcast loads for both tokens;
 //   softmax  once per page: a warp takes a head's 256 scores, so there is one rescaling a page;
@@ -17,6 +22,7 @@
 namespace {
 
 constexpr int DP_THREADS = 128;
+constexpr int DP_GT = 8;           // query heads a CTA takes
 constexpr int DP_S = 256;
 constexpr int DP_SROW = DP_S + 4;  // scores of a head
 constexpr int DP_HOT = 128;        // hot tokens per round
@@ -55,8 +61,8 @@ TQ_DEV float dp_ld(const void* p, size_t i, int dt) {
 }
 
 // GT query heads of one KV head per CTA; grid = (splits, units, head tiles)
-template <int GT>
-__global__ void __launch_bounds__(DP_THREADS, GT == 8 ? 3 : 4) decode_pages_kernel(DecodeArgs a) {
+__global__ void __launch_bounds__(DP_THREADS, 3) decode_pages_kernel(DecodeArgs a) {
+  constexpr int GT = DP_GT;
   constexpr int NP = GT / 2;          // pairs of heads
   constexpr int PROW = GT + 4;        // floats per token of the probabilities
   constexpr int HW = GT / 4;          // heads per warp in the softmax
@@ -453,9 +459,14 @@ __global__ void __launch_bounds__(DP_THREADS, GT == 8 ? 3 : 4) decode_pages_kern
 }  // namespace
 
 void tq_launch_decode_pages(const DecodeArgs& a, int n_units, cudaStream_t st) {
-  // tiles of eight heads (a group of five to seven leaves up to three idle, which costs less than
-  // walking the codes twice).  64 units of seven heads, 700 to 12 000 tokens, two layers: 686 us with
-  // the general kernel and its merge head after head, 376 us here.
-  const dim3 grid(a.ns_cold + a.ns_hot, n_units, (a.g.group + 7) / 8);
-  decode_pages_kernel<8><<<grid, DP_THREADS, 0, st>>>(a);
+  // Tiles of eight heads; a group of five to seven leaves up to three idle, one of nine to fifteen
+  // up to seven of its second tile.  Microseconds a layer, general kernel / this one (K4/V3, bf16; 64
+  // units of 700 to 12 000 tokens, 64 of 6 000, 8 of 32 768, 32 of 900):
+  //   5 heads   252 / 203   264 / 192   191 / 110   39 / 31
+  //   7 heads   254 / 203   266 / 192   192 / 110   39 / 31
+  //   8 heads   310 / 203   311 / 193   232 / 110   52 / 31   (where the general kernel is asked for)
+  //   9 heads   553 / 256   557 / 256   382 / 170   70 / 36
+  //  16 heads   552 / 257   555 / 256   379 / 170   74 / 36
+  const dim3 grid(a.ns_cold + a.ns_hot, n_units, (a.g.group + DP_GT - 1) / DP_GT);
+  decode_pages_kernel<<<grid, DP_THREADS, 0, st>>>(a);
 }

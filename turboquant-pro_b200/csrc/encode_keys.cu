@@ -1,7 +1,7 @@
 // Key encoder for the usual block (256 tokens, up to eight outliers per channel).
 //
 // What the general key encoder (encode.cu) computes, bit for bit.  That kernel was bound by
-// instruction issue (about 170 instructions per element); this one spends about a tenth:
+// instruction issue (150 instructions per element); this one spends 37 (16-bit tokens) or 43:
 //   - a thread owns two neighbouring channels and a segment of the tokens, so 16-bit statistics
 //     are packed two channels to an instruction and a code byte (two channels) is one store;
 //   - the nearest level comes from one table look-up: the range of a channel is cut into 32 bins,
@@ -15,9 +15,11 @@
 //   - outliers: where a block is cut into 32 groups of eight tokens, the k largest magnitudes of a
 //     channel lie in the k groups with the largest maxima (in a few more where maxima are equal),
 //     so only those groups are searched for the k-th magnitude and for the tokens that reach it.
-// Measured (B200): 8 x 16 384 fp16 tokens x 8 heads about 780 us with the general encoder, 241 us
-// here (41 % of it issue slots: two CTAs of an SM do not hide all barriers); 4001 float32 tokens x
-// 32 heads about 300 us and 61 us; the 32 blocks of one flush, alone on the GPU, 16 us.
+// Measured (B200): 8 x 16 384 fp16 tokens x 8 heads about 780 us with the general encoder, 244 us
+// here; 4001 float32 tokens x 32 heads about 300 us and 61 us; the 32 blocks of one flush, alone on the
+// GPU, 16 us.  Counters: 54 % of the issue slots with 16-bit tokens (two CTAs an SM; warps wait for
+// fixed latencies, then for barriers), 39 % with float32 (one CTA an SM, nothing to cover its
+// barriers and its load); DRAM at 17 %.
 // The passes read the block from shared memory, eight tokens an iteration: all loads of an
 // iteration first and its stores last, so that the eight chains of dependent steps overlap.
 #include "encode.cuh"
