@@ -15,8 +15,8 @@
 //   - outliers: where a block is cut into 32 groups of eight tokens, the k largest magnitudes of a
 //     channel lie in the k groups with the largest maxima (in a few more where maxima are equal),
 //     so only those groups are searched for the k-th magnitude and for the tokens that reach it.
-// Measured (B200): 8 x 16 384 fp16 tokens x 8 heads about 780 us with the general encoder, 244 us
-// here; 4001 float32 tokens x 32 heads about 300 us and 61 us; the 32 blocks of one flush, alone on the
+// Measured (B200): 8 x 16 384 fp16 tokens x 8 heads about 780 us with the general encoder, 248 us
+// here; 4001 float32 tokens x 32 heads about 300 us and 62 us; the 32 blocks of one flush, alone on the
 // GPU, 16 us.  Counters: 54 % of the issue slots with 16-bit tokens (two CTAs an SM; warps wait for
 // fixed latencies, then for barriers), 39 % with float32 (one CTA an SM, nothing to cover its
 // barriers and its load); DRAM at 17 %.
