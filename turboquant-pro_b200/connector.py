@@ -37,11 +37,10 @@ def _takes_raw_writes(t) -> bool:
     torch has more to do than store elements (a gradient or a tangent to follow, a transform's
     wrapper, a lazily negated view) or refuses the write (an inference tensor outside its mode)."""
     import torch
-    from torch.autograd import forward_ad
 
     if type(t) is not torch.Tensor or t.requires_grad or t.is_neg() \
             or (t.is_inference() and not torch.is_inference_mode_enabled()) \
-            or forward_ad.unpack_dual(t).tangent is not None:
+            or torch.autograd.forward_ad.unpack_dual(t).tangent is not None:
         return False
     try:
         t.data_ptr()
