@@ -104,6 +104,15 @@ struct Tables {
   uint8_t mean_mask[TQ_D];  // asymmetric NF4: channels that keep their mean (default all)
 };
 
+// Look-up table of the value encoder in encode_values.cu (which explains it); from the boundaries.
+struct ValueTable {
+  bool ok = false;  // the boundaries allow it: ascending, at most one of them in a bin
+  int32_t off[32];
+  uint32_t slack, zero_code;
+  float scale;
+};
+void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable* vt);
+
 struct tq_ctx {
   tq_geom g;
   tq_buffers b;
@@ -124,6 +133,7 @@ struct tq_ctx {
   std::vector<cudaEvent_t> prof_ev;
   float h_centroids[16];
   float h_boundaries[16];
+  ValueTable value_table;
   // tensor maps (opaque 128-byte driver objects) of the two hot rings as 2-D arrays
   // [ring rows][128] of 16-bit elements, for the decode kernel's swizzled tile copies;
   // state 0: not built yet, 1: ready, -1: not available (float32 rings, or no driver entry)

@@ -925,13 +925,6 @@ __global__ void __launch_bounds__(ENCV_HALVES* TQ_D, 2) encode_values_kernel(Enc
 // the page.  The main loop then has three barriers per group and no serial tail.  All waits
 // are bounded.
 // ---------------------------------------------------------------------------------------
-TQ_DEV uint32_t enc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-TQ_DEV uint64_t umma_desc_k_major(uint32_t saddr, uint32_t leading_bytes, uint32_t stride_bytes) {
-  // start address, leading and stride byte offsets in 16-byte units; descriptor version 1;
-  // base offset 0, no swizzle
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((leading_bytes >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((stride_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
 // fp16 x fp16 -> fp32, both operands K-major, M = 128, N = 16
 constexpr uint32_t UMMA_IDESC_M128_N16 = (1u << 4) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
 TQ_DEV void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t accumulate) {
@@ -940,10 +933,6 @@ TQ_DEV void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint3
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
       "l"(desc_a), "l"(desc_b), "r"(UMMA_IDESC_M128_N16), "r"(accumulate)
       : "memory");
-}
-TQ_DEV void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
 }
 TQ_DEV void tmem_ld8(uint32_t taddr, float (&v)[8]) {
   uint32_t r[8];
@@ -1537,7 +1526,8 @@ constexpr int VALUE_ENCODER_DEFAULT = 1;
 int g_value_encoder = VALUE_ENCODER_DEFAULT;  // 0: rotation on mma.sync; 1: on tcgen05.mma
 
 template <int DT>
-int launch_encode_t(const EncodeArgs& a, int sm_count, int device, cudaStream_t st, int* launches) {
+int launch_encode_t(const EncodeArgs& a, const ValueTable& vt, int sm_count, int device,
+                    cudaStream_t st, int* launches) {
   const tq_geom& g = a.g;
   if (a.max_new_blocks > 0) {
     dim3 grid(a.max_new_blocks, g.n_kv_heads, a.seq_count);
@@ -1572,6 +1562,8 @@ int launch_encode_t(const EncodeArgs& a, int sm_count, int device, cudaStream_t 
     }
     static bool attr5_set[16] = {};
     const bool tc5 = g_value_encoder == 1;
+    // whole tiles of 128 tokens and boundaries far enough apart for the table: encode_values.cu
+    const bool tiles = tc5 && g.block_tokens % 128 == 0 && vt.ok;
     if (tc5 && !attr5_set[device & 15]) {
       TQ_CUDA(cudaFuncSetAttribute(encode_values_tc5_kernel<DT, 3>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, ENC5_SMEM));
@@ -1581,19 +1573,23 @@ int launch_encode_t(const EncodeArgs& a, int sm_count, int device, cudaStream_t 
     }
     const int ctas5 = (int)std::min<long>((total + ENC5_PARTS - 1) / ENC5_PARTS, (long)sm_count);
     auto values = [&](const EncodeArgs& av) {
+      if (tiles) return tq_launch_encode_values_tiles(av, vt, sm_count, device, st);
       if (tc5 && g.value_bits == 3)
         encode_values_tc5_kernel<DT, 3><<<ctas5, ENC5_PARTS * TQ_D, ENC5_SMEM, st>>>(av);
       else if (tc5)
         encode_values_tc5_kernel<DT, 4><<<ctas5, ENC5_PARTS * TQ_D, ENC5_SMEM, st>>>(av);
       else
         encode_values_kernel<DT><<<ctas, ENCV_HALVES * TQ_D, ENCV_SMEM, st>>>(av);
+      return (int)TQ_OK;
     };
     if (g.key_mode == TQ_KEYS_POLAR) {
       EncodeArgs ak = a;
       ak.polar_keys_pass = 1;
-      values(ak);
+      const int rc = values(ak);
+      if (rc != TQ_OK) return rc;
     }
-    values(a);
+    const int rc = values(a);
+    if (rc != TQ_OK) return rc;
     *launches += 2;
   }
   // (launched so that it may be scheduled while the kernel before it in the stream drains; it
@@ -1657,9 +1653,9 @@ int tq_launch_encode(tq_ctx* ctx, int layer, int seq_begin, int seq_count, const
   cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, ctx->device);
   int launches = 0;
   switch (ctx->g.kv_dtype) {
-    case TQ_F32: launch_encode_t<TQ_F32>(a, sm_count, ctx->device, st, &launches); break;
-    case TQ_F16: launch_encode_t<TQ_F16>(a, sm_count, ctx->device, st, &launches); break;
-    default: launch_encode_t<TQ_BF16>(a, sm_count, ctx->device, st, &launches); break;
+    case TQ_F32: launch_encode_t<TQ_F32>(a, ctx->value_table, sm_count, ctx->device, st, &launches); break;
+    case TQ_F16: launch_encode_t<TQ_F16>(a, ctx->value_table, sm_count, ctx->device, st, &launches); break;
+    default: launch_encode_t<TQ_BF16>(a, ctx->value_table, sm_count, ctx->device, st, &launches); break;
   }
   ctx->last_launches = launches;
   TQ_CUDA(cudaGetLastError());

@@ -89,3 +89,37 @@ TQ_DEV float f16bits_to_float(uint32_t h) {
 // whether a geometry is of that form.
 bool tq_keys_block_form(const tq_geom& g);
 int tq_launch_encode_keys_block(const EncodeArgs& a, int device, cudaStream_t st);
+
+// Value encoder for blocks of 128 or 256 tokens (encode_values.cu).
+constexpr float VALUE_SPAN = 1023.0f / 1024.0f;  // z = 1 still has a mantissa below 2^23
+int tq_launch_encode_values_tiles(const EncodeArgs& a, const ValueTable& vt, int sm_count, int device,
+                                  cudaStream_t st);
+
+TQ_DEV uint32_t enc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Shared-memory operand of tcgen05.mma, K-major without swizzling: 8 x 8 core matrices of 16-bit
+// values (8 rows of 16 bytes), start address, "leading" offset to the next eight K and "stride"
+// to the next eight rows in 16-byte units; descriptor version 1.
+TQ_DEV uint64_t umma_desc_k_major(uint32_t saddr, uint32_t leading_bytes, uint32_t stride_bytes) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((leading_bytes >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((stride_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+TQ_DEV void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+               : "memory");
+}
+TQ_DEV void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+TQ_DEV void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+TQ_DEV bool mbar_try_wait(uint32_t bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity), "r"(2000u)  // (at most so many nanoseconds a probe)
+      : "memory");
+  return done != 0;
+}
