@@ -32,7 +32,9 @@
 // do it themselves: a batch takes as long as several tiles, and the other warps would wait at the
 // ring of slots.)
 //
-// What bounds it: instruction issue; see the launcher for what it measured.
+// What bounds it (8 x 16 384 tokens x 8 heads, 3 bits, 224 us): the logic pipe and the chains of the epilogue
+// (switched off: 165 us without lists and their recomputation, 124 without codes, products and norms, 83
+// without the copies, too); 42 % of the issue slots, six warps a scheduler.
 #include <algorithm>
 #include <cmath>
 
@@ -56,7 +58,7 @@ constexpr int EV_THREADS = EV_LOADERS + 32 * (EV_EPI_WARPS + EV_REDO_WARPS);
 constexpr int EV_PER_REDO = EV_EPI_WARPS / EV_REDO_WARPS;  // lists a redo warp takes from
 constexpr int EV_LIST = 64;                  // entries of a list (a ring)
 constexpr int EV_PI_BYTES = 2 * TQ_D * TQ_D * 2;
-constexpr int EV_TILE_BYTES = 32768;         // rows of a tile: 128 x 256 or 64 x 512 bytes
+constexpr int EV_TILE_BYTES = 33280;         // rows of a tile: 128 x 256 or 64 x 512 bytes, and the pads
 constexpr int EV_WAIT = 1 << 20;             // probes of a barrier before a wait gives up
 constexpr int EV_POLLS = 1 << 25;            // idle polls before a redo warp gives up
 
@@ -64,6 +66,7 @@ template <int DT>
 struct EvShape {
   static constexpr bool F32 = DT == TQ_F32;
   static constexpr int T = F32 ? 64 : 128;      // tokens of a tile
+  static constexpr int PS = 16 * T + 16;        // bytes from one piece of the rows to the next (padded)
   static constexpr int SLOTS = F32 ? 2 : 4;     // tiles between loader and epilogue
   static constexpr int RAW = F32 ? 2 : 4;       // row buffers (16-bit: they are the operands)
   static constexpr int COLS = F32 ? 128 : 512;  // columns of tensor memory: SLOTS * T
@@ -162,7 +165,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   using T_ = typename Elem<DT>::type;
   using Sh = EvShape<DT>;
   constexpr bool F32 = Sh::F32;
-  constexpr int T = Sh::T, SLOTS = Sh::SLOTS;
+  constexpr int T = Sh::T, PS = Sh::PS, SLOTS = Sh::SLOTS;
   constexpr int EPC = 16 / (int)sizeof(T_), CH = TQ_D / EPC;  // elements of a piece, pieces of a row
   constexpr int VGB = TQ_GROUP_TOK * TQ_D * VB / 8;
   const tq_geom& g = a.g;
@@ -290,24 +293,24 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
           nf.in0 = in0, nf.ring = src.ring;
           nf.n_ring = n_ring, nf.ring0 = ring0;
         }
-        // Piece p of token t goes to (p * T + t) * 16; eight lanes store eight neighbouring tokens, a
-        // warp four pieces of every second (16-bit) or all tokens.
-        constexpr int SPLIT = CH == 16 ? 2 : 1;  // warps that share four pieces
-        const int p = (warp / SPLIT) * 4 + (lane >> 3), t8 = (warp % SPLIT) * 8 + (lane & 7);
-        uint8_t* buf = sh.tile[i % Sh::RAW] + (p * T + t8) * 16;
+        // Piece p of token t goes to p * PS + t * 16; a half warp (float32: a warp) copies a whole row.
+        // (The pad spreads the pieces of a row over the banks.)
+        constexpr int RPI = EV_LOADERS / CH;  // rows of an iteration
+        const int p = tl % CH, t8 = tl / CH;
+        uint8_t* buf = sh.tile[i % Sh::RAW] + p * PS + t8 * 16;
         if (rows_aligned && n_ring == 0) {
           const T_* row = in0 + (int64_t)t8 * src.tok_stride + p * EPC;
-          const int64_t next = (int64_t)(8 * SPLIT) * src.tok_stride;
+          const int64_t next = (int64_t)RPI * src.tok_stride;
           const uint32_t to = enc_smem(buf);
 #pragma unroll
-          for (int it = 0; it < T / (8 * SPLIT); ++it) {
-            ev_cp16(to + it * (128 * SPLIT), row);
+          for (int it = 0; it < T / RPI; ++it) {
+            ev_cp16(to + it * (16 * RPI), row);
             row += next;
           }
         } else {
 #pragma unroll 1
-          for (int it = 0; it < T / (8 * SPLIT); ++it, buf += 128 * SPLIT) {
-            const int t = t8 + it * 8 * SPLIT;
+          for (int it = 0; it < T / RPI; ++it, buf += 16 * RPI) {
+            const int t = t8 + it * RPI;
             int slot = ring0 + t;
             slot -= slot >= src.cap ? src.cap : 0;
             const T_* row = (t < n_ring ? (const T_*)src.ring + (size_t)slot * TQ_D
@@ -338,8 +341,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
       const uint64_t a_hi0 = umma_desc_k_major(enc_smem(sh.pi), 2048, 128);
       const uint64_t a_lo0 = umma_desc_k_major(enc_smem(sh.pi) + EV_PI_BYTES / 2, 2048, 128);
       const uint64_t b0 = umma_desc_k_major(
-          enc_smem(sh.tile[F32 ? 2 + i % 2 : i % 4]), T * 16, 128);
-      constexpr uint64_t KA = 4096 >> 4, KB = 2 * T * 16 >> 4;  // a step of 16 input channels
+          enc_smem(sh.tile[F32 ? 2 + i % 2 : i % 4]), PS, 128);
+      constexpr uint64_t KA = 4096 >> 4, KB = 2 * PS >> 4;  // a step of 16 input channels
 #pragma unroll
       for (int kb = 0; kb < 8; ++kb) {  // the small products first (see value_slack)
         ev_mma(d, a_lo0 + kb * KA, b0 + kb * KB, idesc, kb > 0);
@@ -375,7 +378,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
         // unfused one does - above the denormals: see below)
 #pragma unroll 4
         for (int p = 0; p < CH; ++p) {
-          const uint2 v = *(const uint2*)(buf + p * T * 16);
+          const uint2 v = *(const uint2*)(buf + p * PS);
           ev_sq2(r[0], ev_pair<DT>(v.x));
           ev_sq2(r[1], ev_pair<DT>(v.y));
         }
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
           any = 0u;
           r[0] = r[1] = make_float2(0.0f, 0.0f);
           for (int p = 0; p < CH; ++p) {
-            const uint2 v = *(const uint2*)(buf + p * T * 16);
+            const uint2 v = *(const uint2*)(buf + p * PS);
             any |= (v.x | v.y) & 0x7fff7fffu;
             const float2 f0 = ev_pair<DT>(v.x), f1 = ev_pair<DT>(v.y);
             r[0].x = __fadd_rn(r[0].x, __fmul_rn(f0.x, f0.x));
@@ -417,10 +420,10 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
         sync();
         // four threads a token: accumulators 2u and 2u + 1, elements 8p + 2u and 8p + 2u + 1 of its row
         const int t = 8 * warp + ((lane >> 1) & 7), u = 2 * (lane >> 4) + (lane & 1);
-        const uint8_t* buf = sh.tile[i % Sh::RAW] + ((u >> 1) * T + t) * 16 + (u & 1) * 8;
+        const uint8_t* buf = sh.tile[i % Sh::RAW] + (u >> 1) * PS + t * 16 + (u & 1) * 8;
         float2 x[CH / 2], r;
 #pragma unroll
-        for (int p = 0; p < CH / 2; ++p) x[p] = *(const float2*)(buf + p * 2 * T * 16);
+        for (int p = 0; p < CH / 2; ++p) x[p] = *(const float2*)(buf + p * 2 * PS);
         uint32_t any = 0u;  // an element that is not zero
 #pragma unroll
         for (int p = 0; p < CH / 2; ++p) {
@@ -440,8 +443,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
         uint8_t* op = sh.tile[2 + i % 2] + t * 16 + u * 4;
 #pragma unroll
         for (int p = 0; p < CH / 2; ++p)
-          ev_split<DT>(make_float2(x[p].x * up, x[p].y * up), *(uint32_t*)(op + p * T * 16),
-                       *(uint32_t*)(op + EV_TILE_BYTES / 2 + p * T * 16));
+          ev_split<DT>(make_float2(x[p].x * up, x[p].y * up), *(uint32_t*)(op + p * PS),
+                       *(uint32_t*)(op + EV_TILE_BYTES / 2 + p * PS));
         if (u == 0) {
           sh.info[i & 3].nrm_dst[t] = nrm;
           sh.norm[slot][t] = nrm;
@@ -669,7 +672,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
           if (lane == 0) atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
           break;
         }
-        __nanosleep(1000);
+        __nanosleep(2000);
         continue;
       }
       if (total == 0) break;  // (and nothing more to come)
@@ -741,6 +744,9 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   }
 }
 
+// Microseconds of the value encoder, groups of 16 tokens (encode_values_tc5_kernel) / this one: 8 x 16 384 fp16
+// tokens x 8 heads, 3 bits, 566 / 224; bf16, 4 bits, 612 / 247; 4 001 float32 tokens x 32 heads, 4 bits, 92 / 62;
+// 3 333 bf16 tokens x 8 heads, 4 bits, 33 / 24; 4 x 1 010, 3 bits, 32 / 20.
 template <int DT, int VB>
 int launch_tiles(const EncodeArgs& a, const ValueTable& vt, int sm_count, int device, cudaStream_t st) {
   static bool attr_set[16] = {};  // per device: the attribute belongs to the device's context
