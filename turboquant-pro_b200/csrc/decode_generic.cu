@@ -435,8 +435,9 @@ __global__ void __launch_bounds__(WARPS * 32) decode_generic_kernel(DecodeArgs a
 // Split-K combine: one CTA per (seq, KV head) and query head of its group.  Cold partials are summed
 // in code space and un-rotated once (acc @ Pi); hot partials are already in the original basis.
 // Bound by latency, so the heads of a group do not take turns in one CTA (64 units of seven heads,
-// 6 000 tokens: 51 us that way, 12 us here; of three heads 43 and 11 us; 8 units of 32 768 tokens and
-// seven heads 96 and 18 us; between events around the launch).
+// 6 000 tokens: 51 us that way), and what it reads comes in as few trips to memory as the registers
+// hold: 64 units of three heads 11.3 us with a trip per four partials, 10.2 us this way; 32 units
+// of 900 tokens 11.2 and 9.4 us (between events around the launch).
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(TQ_D) combine_kernel(DecodeArgs a) {
   const tq_geom& g = a.g;
@@ -447,24 +448,40 @@ __global__ void __launch_bounds__(TQ_D) combine_kernel(DecodeArgs a) {
   __shared__ float cs[TQ_D];
   const float* base = a.partials + ((size_t)unit * g.max_splits * G + gg) * TQ_PART_STRIDE;
   const size_t stride = (size_t)G * TQ_PART_STRIDE;
+  // the states and the first sums in one trip to memory
+  __shared__ float s_m[TQ_D], s_l[TQ_D], s_w[TQ_D];
+  constexpr int FIRST = 32;
+  float x[FIRST];
+  if (e < ns) {
+    s_m[e] = base[e * stride];
+    s_l[e] = base[e * stride + 1];
+  }
+#pragma unroll
+  for (int s = 0; s < FIRST; ++s) x[s] = s < ns ? base[s * stride + 2 + e] : 0.0f;
+  __syncthreads();
   float M = -INFINITY;
 #pragma unroll 8
-  for (int s = 0; s < ns; ++s) M = fmaxf(M, base[s * stride]);
+  for (int s = 0; s < ns; ++s) M = fmaxf(M, s_m[s]);
+  if (e < ns) s_w[e] = s_m[e] > -INFINITY ? __expf(s_m[e] - M) : 0.0f;
+  __syncthreads();
   float L = 0.0f, C = 0.0f, Hh = 0.0f;
-#pragma unroll 4
-  for (int s = 0; s < ns; ++s) {
-    const float* pp = base + s * stride;
-    const float w = pp[0] > -INFINITY ? __expf(pp[0] - M) : 0.0f;
-    L += pp[1] * w;
+  auto add = [&](int s, float y) {
+    const float v = s_m[s] > -INFINITY ? y * s_w[s] : 0.0f;  // (an empty partial has no sums)
+    L += s_l[s] * s_w[s];
     if (s < a.ns_cold)
-      C += pp[2 + e] * w;
+      C += v;
     else
-      Hh += pp[2 + e] * w;
-  }
+      Hh += v;
+  };
+#pragma unroll
+  for (int s = 0; s < FIRST; ++s)
+    if (s < ns) add(s, x[s]);
+#pragma unroll 32
+  for (int s = FIRST; s < ns; ++s) add(s, base[s * stride + 2 + e]);
   cs[e] = C;
   __syncthreads();
   float o = 0.0f;
-#pragma unroll 16
+#pragma unroll 32
   for (int d = 0; d < TQ_D; ++d) o += cs[d] * a.tables->pi[d * TQ_D + e];
   const size_t row = (size_t)seq * g.n_q_heads + head * G + gg;
   const float val = o + Hh;
@@ -506,12 +523,9 @@ void launch_generic(const DecodeArgs& a, int n_units, cudaStream_t st) {
 
 // Groups of five and more on 256-token blocks: decode_pages.cu, also where the caller asks for the
 // general kernel.  Everything else here.
-void launch_generic_any(const DecodeArgs& a, int n_units, cudaStream_t st) {
+int launch_generic_any(const DecodeArgs& a, int n_units, int sm_count, cudaStream_t st) {
   const tq_geom& g = a.g;
-  if (tq_decode_pages_form(g)) {
-    tq_launch_decode_pages(a, n_units, st);
-    return;
-  }
+  if (tq_decode_pages_form(g)) return tq_launch_decode_pages(a, sm_count, st);
   int gt = g.group >= 8 ? 8 : (g.group > 2 ? 4 : (g.group > 1 ? 2 : 1));
   switch (gt) {
     case 1: launch_generic<1>(a, n_units, st); break;
@@ -519,6 +533,7 @@ void launch_generic_any(const DecodeArgs& a, int n_units, cudaStream_t st) {
     case 4: launch_generic<4>(a, n_units, st); break;
     default: launch_generic<8>(a, n_units, st); break;
   }
+  return TQ_OK;
 }
 
 }  // namespace
@@ -568,11 +583,13 @@ int tq_launch_decode(tq_ctx* ctx, int layer, const void* q, int q_dtype, int blo
   // split counts from the longest sequence of the layer: about two pages (or eight hot
   // groups) per CTA, bounded by the scratch slots
   int max_nb = 0, max_hot = 0;
+  long total_nb = 0;
   for (int s = 0; s < g.n_seqs; ++s) {
     int n = ctx->len[(size_t)layer * g.n_seqs + s];
     int nb = n_cold_blocks(n, g.hot_window, g.block_tokens);
     int b1 = block_end < 0 ? nb : std::min(block_end, nb);
     max_nb = std::max(max_nb, std::max(b1 - std::min(block_begin, nb), 0));
+    total_nb += std::max(b1 - std::min(block_begin, nb), 0);
     max_hot = std::max(max_hot, n - nb * g.block_tokens);
   }
   int n_units = g.n_seqs * g.n_kv_heads;
@@ -582,20 +599,29 @@ int tq_launch_decode(tq_ctx* ctx, int layer, const void* q, int q_dtype, int blo
   int hot_groups = with_hot ? (max_hot + TQ_GROUP_TOK - 1) / TQ_GROUP_TOK : 0;
   int ns_hot = hot_groups > 0 ? std::min(std::min(hot_groups, std::max(1, want / 4)), 16) : 0;
   int ns_cold = max_nb > 0 ? std::min(std::min(max_nb, want), g.max_splits - ns_hot) : 0;
+  if (tq_decode_pages_form(g)) {
+    // the page kernel cuts the list of all pages into equal shares: room for the partials of the longest
+    // sequence; the window in rounds of 64 tokens
+    ns_hot = with_hot ? std::min((max_hot + 63) / 64, 8) : 0;
+    const long groups = 3l * sm_count;
+    const long share = std::max((total_nb * g.n_kv_heads * ((g.group + 7) / 8) + groups - 1) / groups, 1l);
+    ns_cold = max_nb > 0 ? (int)std::min<long>(std::max((max_nb - 1) / share + 3, 2l), g.max_splits - ns_hot) : 0;
+  }
   if (ns_cold + ns_hot == 0) ns_hot = 1;  // empty layer: the kernels still write zeros
   a.ns_cold = ns_cold;
   a.ns_hot = ns_hot;
 
   cudaEvent_t e0 = tq_prof_event(ctx, 0), e1 = tq_prof_event(ctx, 1), e2 = tq_prof_event(ctx, 2);
   if (e0) cudaEventRecord(e0, st);
-  launch_generic_any(a, n_units, st);
+  rc = launch_generic_any(a, n_units, sm_count, st);
+  if (rc != TQ_OK) return rc;
   if (e1) cudaEventRecord(e1, st);
   combine_kernel<<<dim3(n_units, g.group), TQ_D, 0, st>>>(a);
   if (e2) {
     cudaEventRecord(e2, st);
     tq_prof_commit(ctx);
   }
-  ctx->last_launches = 2;
+  ctx->last_launches = 1 + (tq_decode_pages_form(g) ? (g.n_seqs + TQ_PAGES_SEQS - 1) / TQ_PAGES_SEQS : 1);
   ctx->last_kernel = TQ_KERNEL_GENERAL;
   TQ_CUDA(cudaGetLastError());
   return TQ_OK;
@@ -690,13 +716,17 @@ extern "C" int32_t tq_decode_static_scratch(tq_ctx* ctx, int32_t layer, const vo
   const int n_units = g.n_seqs * g.n_kv_heads;
   int ns_hot = max_hot > 0 ? std::min((max_hot + 127) / 128, 2) : 0;
   int ns_cold = max_nb > 0 ? std::min(max_nb, TQ_STATIC_SLOTS - ns_hot) : 0;
+  if (tq_decode_pages_form(g) && ns_cold > 0) ns_cold = TQ_STATIC_SLOTS - ns_hot;
   if (ns_cold + ns_hot == 0) ns_hot = 1;  // empty layer: the kernels still write zeros
   a.ns_cold = ns_cold;
   a.ns_hot = ns_hot;
 
-  launch_generic_any(a, n_units, st);
+  int sm_count = 148;
+  cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, ctx->device);
+  const int rc = launch_generic_any(a, n_units, sm_count, st);
+  if (rc != TQ_OK) return rc;
   combine_kernel<<<dim3(n_units, g.group), TQ_D, 0, st>>>(a);
-  ctx->last_launches = 2;
+  ctx->last_launches = 1 + (tq_decode_pages_form(g) ? (g.n_seqs + TQ_PAGES_SEQS - 1) / TQ_PAGES_SEQS : 1);
   ctx->last_kernel = TQ_KERNEL_GENERAL;
   ctx->last_q_dtype = q_dtype;
   TQ_CUDA(cudaGetLastError());

@@ -23,10 +23,11 @@ struct DecodeArgs {
 };
 
 // Query groups of five and more on 256-token blocks (per-channel keys) take the page kernel; its times
-// beside the general kernel's stand at its launch.  Distance from 64 bits over 40 to 12 000 tokens,
-// general kernel / page kernel: 1.18e-6 / 1.11e-6 at five heads, 1.13 / 1.06 at seven, 1.11 / 1.06 at
-// nine, 1.12 / 1.06 at sixteen.  (At three heads it came out a tenth further away: not taken.)
+// beside the general kernel's stand at its launch.  Distance from 64 bits over 30 to 12 000 tokens: 8.9e-7
+// at five heads, 7.3e-7 at seven, 8.9e-7 at twelve; with plain float32 multiply-adds in place of the split
+// products 1.11e-6, 9.2e-7 and 9.0e-7, the general kernel about 1.12e-6.
 TQ_HD bool tq_decode_pages_form(const tq_geom& g) {
   return g.block_tokens == 256 && g.key_mode != TQ_KEYS_POLAR && g.group > 4;
 }
-void tq_launch_decode_pages(const DecodeArgs& a, int n_units, cudaStream_t st);
+constexpr int TQ_PAGES_SEQS = 2048;  // sequences a launch of the page kernel covers
+int tq_launch_decode_pages(const DecodeArgs& a, int sm_count, cudaStream_t st);

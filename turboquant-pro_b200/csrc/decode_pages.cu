@@ -1,31 +1,81 @@
-// Decode-on-codes attention in float32 for 256-token blocks and query groups the tensor-core kernel
-// has no tile for (5, 6, 7 and 9 to 16 query heads per KV head), and for larger groups wherever the
-// general-shape kernel is asked for.  Same arithmetic as decode_generic.cu: float32 products and sums
-// throughout; the partials have its layout and go through its combine kernel.
+// Decode-on-codes attention to float32 accuracy for 256-token blocks and query groups the tensor-core
+// kernel has no tile for (5, 6, 7 and 9 to 16 query heads per KV head), and for larger groups wherever
+// the general-shape kernel is asked for.  The partials have the layout of decode_generic.cu and go
+// through its combine kernel.
 //
-// Bound by latency, not by issue.  Counters of one launch (160 units of seven heads, 700 to 12 000
-// tokens, 422 us): 32 % of the issue slots, 2.5 warps per scheduler of which 0.4 can issue; of 7.9
-// cycles between two instructions of a warp 3.6 wait for global memory (codes, scales, norms and outlier
-// lists are fetched where they are used, between the page's four barriers); and the splits are uneven, the
-// busiest SM works 822 000 cycles, the average one 633 000.  168 registers hold it at three CTAs an
-// SM, with 40 bytes spilled.  decode_generic.cu looks every code up once per tile of four heads, a
-// 16-token group at a time; here a code is looked up once for eight heads and feeds packed
-// multiply-adds (two heads an instruction), sixteen instructions per code and lane in all:
-//   scores   a lane owns two tokens and walks their channels; the weights w = q * scale of a channel
-//            lie side by side for the heads, two broadcast loads for both tokens;
-//   softmax  once per page: a warp takes a head's 256 scores, so there is one rescaling a page;
-//   values   a warp takes half the channels of every second 16-token group (one 12- or 16-byte load
-//            per lane), its tokens' probabilities come as four-head vectors.
-// The uncompressed window: a thread per token for the scores, a thread per channel for the values.
+// The products run on mma.sync tiles (m16n8k16, eight query heads across) with every float32 operand
+// split into two fp16 parts, x = hi + lo: 22 bits and the sign, scaled by powers of two so that lo keeps
+// its bits.  hi * hi + hi * lo + lo * hi leaves out 2^-24 of a term; the three products of a 16-deep
+// step start from zero and are added up in float32 registers with ordinary rounding (a chain
+// inside the tensor cores would truncate at every step).
+//
+// Persistent CTAs of three groups of four warps, one CTA an SM.  The pages of all sequences, heads and
+// head tiles form one list that is cut into equal shares, one per group, so ragged batches balance;
+// where a share leaves a (sequence, head) the group writes a partial.  A warp takes a strip of 64 tokens
+// of each page of the share and works on it alone, without barriers: it copies what it needs of the
+// page (codes, scales, outlier slots; value codes, norms) into its own piece of shared memory with
+// cp.async, the key half of the next page while it works on the values of this one and the other way
+// round (loading them where they are used left the warps waiting most of the time).
+//   weights  w = q * scale as B fragments of its own (a lane forms the 32 weights it holds), the
+//            zero-points' share of the score beside them;
+//   scores   a byte of codes (two channels) becomes the hi and lo pairs by one 8-byte look-up in a
+//            table with a copy per lane of a half warp: no bank conflicts, no arithmetic;
+//   softmax  once per strip, in registers: a lane has two heads of two tokens a tile;
+//   values   probability times norm, split, goes from the score tile's layout to the value tile's by
+//            8x8 transposes; two tokens' codes of a channel are one look-up, as above.
+// Outliers come from the page's own list by token (four fixed slots, then the overflow entries).
+//
+// The uncompressed window follows, in splits of its own: rounds of 64 tokens, their rows copied into
+// shared memory (stride padded by 16 bytes: a thread per token reads them without conflicts), two
+// threads a token for the scores, a thread per channel for the values, in packed float32 multiply-adds.
 #include "decode_generic.cuh"
 
 namespace {
 
-constexpr int DP_THREADS = 128;
-constexpr int DP_GT = 8;           // query heads a CTA takes
+constexpr int DP_GROUPS = 3;
+constexpr int DP_GTH = 128;          // threads of a group
+constexpr int DP_THREADS = DP_GROUPS * DP_GTH;
+constexpr int DP_GT = 8;             // query heads of a tile
 constexpr int DP_S = 256;
-constexpr int DP_SROW = DP_S + 4;  // scores of a head
-constexpr int DP_HOT = 128;        // hot tokens per round
+constexpr int DP_STRIP = 64;         // tokens of a page a warp takes
+constexpr int DP_HOT = 64;           // hot tokens per round
+constexpr int DP_SROW = DP_HOT + 4;  // scores of a head
+constexpr int DP_PROW = DP_GT + 4;   // floats per token of the probabilities
+constexpr int DP_SEQS = TQ_PAGES_SEQS;
+
+// A warp's strip of a page.
+template <int VB>
+struct alignas(16) DpStrip {
+  uint8_t keys[DP_STRIP * TQ_D / 2];
+  uint16_t delta[TQ_ELL_SLOTS][DP_STRIP];
+  uint8_t col[TQ_ELL_SLOTS][DP_STRIP];
+  float scale[4][36], mean[4][36];  // 32 channels a row (the pad spreads a lane's rows over the banks)
+  PageHeader hdr;
+  uint32_t ovf[TQ_OVF_CAP];
+  uint8_t values[DP_STRIP * TQ_D * VB / 8];
+  float norms[DP_STRIP];
+};
+struct DpHot {
+  float s[DP_GT][DP_SROW];
+  float p[DP_HOT][DP_PROW];
+  alignas(16) uint8_t rows[DP_HOT * (TQ_D * 4 + 16)];
+};
+
+template <int VB>
+struct DpShared {
+  static constexpr int NV = VB == 4 ? 256 : 64;
+  uint2 lutk[256][16], lutv[NV][16];  // (hi pair, lo pair) of two codes, a copy per lane mod 16
+  union {
+    DpStrip<VB> strip[4];
+    DpHot hot;
+  } group[DP_GROUPS];
+  float corr[DP_GROUPS][4][32][DP_GT];  // per warp: outlier corrections of 32 tokens; the merge area
+  float q[DP_GROUPS][TQ_D][DP_GT];      // row q_row(d): channel d
+  float m[DP_GROUPS][4][DP_GT], l[DP_GROUPS][4][DP_GT], f[DP_GROUPS][DP_GT];
+  float grid[16], cent[16];
+  int cum[DP_SEQS + 1];                 // pages of the sequences before each one (a head tile's worth)
+  int scan[DP_THREADS / 32], most[DP_THREADS / 32];
+};
 
 TQ_DEV unsigned long long dp_pack(float a, float b) {
   unsigned long long r;
@@ -60,413 +110,765 @@ TQ_DEV float dp_ld(const void* p, size_t i, int dt) {
   return __bfloat162float(((const __nv_bfloat16*)p)[i]);
 }
 
-// GT query heads of one KV head per CTA; grid = (splits, units, head tiles)
-__global__ void __launch_bounds__(DP_THREADS, 3) decode_pages_kernel(DecodeArgs a) {
+TQ_DEV uint32_t dp_h2(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *(const uint32_t*)&h;
+}
+// a pair of floats as fp16 pairs, hi + lo
+TQ_DEV void dp_split(float a, float b, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(a, b);
+  const float2 f = __half22float2(h);
+  hi = *(const uint32_t*)&h;
+  lo = dp_h2(a - f.x, b - f.y);
+}
+TQ_DEV uint2 dp_lut(uint32_t addr) {  // (the tables never change: not volatile)
+  uint2 v;
+  asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+TQ_DEV void dp_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1,
+                   const float (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]),
+        "f"(c[2]), "f"(c[3]));
+}
+// d = a * b of one 16-deep step, the small products first
+TQ_DEV void dp_product(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4],
+                       const uint32_t (&bh)[2], const uint32_t (&bl)[2]) {
+  const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  dp_mma(d, al, bh[0], bh[1], zero);
+  dp_mma(d, ah, bl[0], bl[1], d);
+  dp_mma(d, ah, bh[0], bh[1], d);
+}
+TQ_DEV uint32_t dp_transpose(uint32_t v) {  // of an 8x8 matrix of 16-bit elements, a row per four lanes
+  uint32_t o;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(o) : "r"(v));
+  return o;
+}
+// 2^(top - floor(log2 x)), the power of two that takes x to [2^top, 2^(top + 1)); and its inverse.  Zero,
+// denormals, infinities and NaN count as the nearest ordinary exponent.
+TQ_DEV float dp_lift(float x, int top, float& inverse) {
+  const int e = min(max((int)(__float_as_uint(x) >> 23 & 255u), 32), 254);
+  inverse = __int_as_float((e - top) << 23);
+  return __int_as_float((254 + top - e) << 23);
+}
+TQ_DEV void dp_cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+TQ_DEV void dp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// sequences seq0 .. seq0 + n_seqs - 1 of the layer
+template <int VB>
+__global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs a, int seq0, int n_seqs) {
   constexpr int GT = DP_GT;
   constexpr int NP = GT / 2;          // pairs of heads
-  constexpr int PROW = GT + 4;        // floats per token of the probabilities
-  constexpr int HW = GT / 4;          // heads per warp in the softmax
+  constexpr int VGB = TQ_GROUP_TOK * TQ_D * VB / 8;
+  extern __shared__ __align__(128) uint8_t dp_smem[];
+  DpShared<VB>& sh = *(DpShared<VB>*)dp_smem;
   const tq_geom& g = a.g;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int split = blockIdx.x, unit = blockIdx.y, gt = blockIdx.z;
-  const int seq = unit / g.n_kv_heads, head = unit % g.n_kv_heads;
-  const int G = g.group, vb = g.value_bits;
-  const int N = a.seq_len[a.layer * g.n_seqs + seq];
-  const int nb = n_cold_blocks(N, g.hot_window, DP_S);
-  const bool cold = split < a.ns_cold;
+  const int tid = threadIdx.x, lane = tid & 31, gi = tid / DP_GTH, gtid = tid % DP_GTH, warp = gtid >> 5;
+  const int r = lane >> 2, c = lane & 3;
+  const int G = g.group, H = g.n_kv_heads, tiles = (G + GT - 1) / GT;
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + gi), "n"(DP_GTH) : "memory"); };
+  float(*q_s)[GT] = sh.q[gi];
 
-  __shared__ __align__(16) float q_s[TQ_D][GT], w_s[TQ_D][GT];
-  __shared__ float s_s[GT][DP_SROW];  // outlier corrections, then scores
-  __shared__ __align__(16) float p_s[DP_S][PROW];
-  __shared__ float bias_w[4][GT], f_s[GT];
-  __shared__ float nf4_s[16], cent_s[16];
+  // ---- tables, the list of pages ---------------------------------------------------------------
   if (tid < 16) {
-    nf4_s[tid] = a.tables->grid[tid];
-    cent_s[tid] = a.tables->centroids[tid];
+    sh.grid[tid] = a.tables->grid[tid];
+    sh.cent[tid] = a.tables->centroids[tid];
   }
+  auto pages_of = [&](int s, int& b0) -> int {
+    const int nb = n_cold_blocks(a.seq_len[a.layer * g.n_seqs + seq0 + s], g.hot_window, DP_S);
+    b0 = min(a.block_begin, nb);
+    return (a.block_end < 0 ? nb : min(a.block_end, nb)) - b0;
+  };
+  int most = 0;  // pages of the longest sequence
+  {
+    // thread t takes sequences t * per .. + per - 1: a scan over the threads
+    const int per = (n_seqs + DP_THREADS - 1) / DP_THREADS;
+    int sum = 0, b0;
+    for (int s = tid * per; s < min((tid + 1) * per, n_seqs); ++s) {
+      const int n = pages_of(s, b0);
+      sh.cum[s + 1] = n;
+      sum += n;
+      most = max(most, n);
+    }
+    int incl = sum;
 #pragma unroll
-  for (int gg = 0; gg < GT; ++gg) {
-    const int qh = gt * GT + gg;
-    q_s[tid][gg] = qh < G ? dp_ld(a.q, ((size_t)seq * g.n_q_heads + head * G + qh) * TQ_D + tid,
-                                  a.q_dtype)
-                          : 0.0f;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 31) sh.scan[tid >> 5] = incl;
+    if (lane == 0) sh.most[tid >> 5] = most;
+    __syncthreads();
+    int before = incl - sum;
+    for (int w = 0; w < DP_THREADS / 32; ++w) {
+      before += w < tid >> 5 ? sh.scan[w] : 0;
+      most = max(most, sh.most[w]);
+    }
+    if (tid == 0) sh.cum[0] = 0;
+    for (int s = tid * per; s < min((tid + 1) * per, n_seqs); ++s) {
+      before += sh.cum[s + 1];
+      sh.cum[s + 1] = before;
+    }
   }
-  float m_run[HW], l_run[HW];  // of heads warp * HW + i, the same in every lane
+  float inv_k, inv_v;
+  {  // entries scaled to below 2^8
+    float max_k = 0.0f, max_v = 0.0f;
 #pragma unroll
-  for (int i = 0; i < HW; ++i) {
-    m_run[i] = -INFINITY;
-    l_run[i] = 0.0f;
+    for (int i = 0; i < 16; ++i) {
+      max_k = fmaxf(max_k, fabsf(sh.grid[i]));
+      max_v = fmaxf(max_v, fabsf(sh.cent[i]));
+    }
+    const float up_k = dp_lift(max_k, 7, inv_k), up_v = dp_lift(max_v, 7, inv_v);
+    for (int e = tid; e < 256 + DpShared<VB>::NV; e += DP_THREADS) {
+      uint2 w;
+      uint4* dst;
+      if (e < 256) {
+        dp_split(sh.grid[e & 15] * up_k, sh.grid[e >> 4] * up_k, w.x, w.y);
+        dst = (uint4*)sh.lutk[e];
+      } else {
+        const int b = e - 256;
+        dp_split(sh.cent[b & (VB == 4 ? 15 : 7)] * up_v, sh.cent[b >> VB] * up_v, w.x, w.y);
+        dst = (uint4*)sh.lutv[b];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dst[(i + lane) & 7] = make_uint4(w.x, w.y, w.x, w.y);
+    }
   }
   __syncthreads();
 
-  // the softmax of a round's scores: probabilities times `wgt`, and the factor for what was
-  // accumulated before
-  auto softmax = [&](int n_tok, auto wgt) {
+  // A sequence with n pages has n pages in the list for each of its heads and head tiles ("rows" of n
+  // pages).  Shares of `share` pages; a row meets at most (n - 2) / share + 2 of them, which has to fit its
+  // ns_cold partials (at least two).
+  const int rows_per_seq = H * tiles, n_groups = gridDim.x * DP_GROUPS;
+  const long total = (long)sh.cum[n_seqs] * rows_per_seq;
+  int share = (int)((total + n_groups - 1) / n_groups);
+  share = max(share, a.ns_cold > 2 ? (most + a.ns_cold - 4) / (a.ns_cold - 2) : most);
+  share = max(share, 1);
+
+  // the query rows of a tile
+  auto load_q = [&](int unit, int gt) {
+    const int seq = unit / H, head = unit - seq * H;
 #pragma unroll
-    for (int i = 0; i < HW; ++i) {
-      const int gg = warp * HW + i;
-      float mx = -INFINITY;
-      for (int t = lane; t < n_tok; t += 32) mx = fmaxf(mx, s_s[gg][t]);
-      __syncwarp();
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float m_new = fmaxf(m_run[i], mx);
-      const bool any = m_new > -INFINITY;
-      const float f = any ? __expf(m_run[i] - m_new) : 1.0f;
-      float sum = 0.0f;
-      for (int t = lane; t < n_tok; t += 32) {
-        const float p = any ? __expf(s_s[gg][t] - m_new) : 0.0f;
-        sum += p;
-        p_s[t][gg] = p * wgt(t);
+    for (int gg = 0; gg < GT; ++gg) {
+      const int qh = gt * GT + gg;
+      q_s[q_row(gtid)][gg] = qh < G ? dp_ld(a.q, ((size_t)seq * g.n_q_heads + head * G + qh) * TQ_D + gtid,
+                                            a.q_dtype)
+                                    : 0.0f;
+    }
+  };
+  auto slot_of = [&](int unit, int gt, int slot) -> float* {
+    return a.partials + (((size_t)unit * g.max_splits + slot) * G + gt * GT) * TQ_PART_STRIDE;
+  };
+  auto mark_empty = [&](int unit, int gt, int first, int end) {  // partials that hold nothing
+    for (int i = gtid; i < (end - first) * GT; i += DP_GTH)
+      if (gt * GT + i % GT < G) {
+        float* pp = slot_of(unit, gt, first + i / GT) + (i % GT) * TQ_PART_STRIDE;
+        pp[0] = -INFINITY;
+        pp[1] = 0.0f;
       }
-      __syncwarp();
+  };
+  if (a.ns_cold > 0)
+    for (int s = blockIdx.x * DP_GROUPS + gi; s < n_seqs; s += n_groups)
+      if (sh.cum[s + 1] == sh.cum[s])
+        for (int row = 0; row < rows_per_seq; ++row)
+          mark_empty((seq0 + s) * H + row / tiles, row % tiles, 0, a.ns_cold);
+
+  // ---- cold pages -----------------------------------------------------------------------------
+  // a page of the list: sequence, row, page of the row, pages of the row
+  struct Pos {
+    int seq, row, page, n;
+  };
+  auto advance = [&](Pos& p) {  // to the next page
+    if (++p.page < p.n) return;
+    p.page = 0;
+    if (++p.row < rows_per_seq) return;
+    p.row = 0;
+    do {
+      ++p.seq;
+    } while (p.seq < n_seqs && sh.cum[p.seq + 1] == sh.cum[p.seq]);
+    p.n = p.seq < n_seqs ? sh.cum[p.seq + 1] - sh.cum[p.seq] : 1;
+  };
+  const uint32_t lutk = (uint32_t)__cvta_generic_to_shared(&sh.lutk[0][lane & 15]);
+  const uint32_t lutv = (uint32_t)__cvta_generic_to_shared(&sh.lutv[0][lane & 15]);
+  DpStrip<VB>& st = sh.group[gi].strip[warp];
+  float(*corr)[GT] = sh.corr[gi][warp];
+  const int t0 = DP_STRIP * warp;  // first token of this warp's strip
+
+  auto page_at = [&](const Pos& p) -> const uint8_t* {
+    int b0;
+    pages_of(p.seq, b0);
+    return a.pages + page_offset(g, a.layer, seq0 + p.seq, p.row / tiles, b0 + p.page);
+  };
+  auto copy_keys = [&](const uint8_t* page) {
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      l_run[i] = l_run[i] * f + sum;
-      m_run[i] = m_new;
-      if (lane == 0) f_s[gg] = f;
+    for (int i = 0; i < 8; ++i)
+      dp_cp16(st.keys + (32 * i + lane) * 16, page + t0 * (TQ_D / 2) + (32 * i + lane) * 16);
+    const uint8_t* ed = page + g.hdr_off + TQ_ELL_OFF;      // 8 pieces a slot
+    const uint8_t* ec = page + g.hdr_off + TQ_ELL_COL_OFF;  // 4 pieces a slot
+    dp_cp16((uint8_t*)st.delta + lane * 16, ed + (lane >> 3) * (DP_S * 2) + t0 * 2 + (lane & 7) * 16);
+    if (lane < 16) dp_cp16((uint8_t*)st.col + lane * 16, ec + (lane >> 2) * DP_S + t0 + (lane & 3) * 16);
+    dp_cp16(&st.scale[lane >> 3][(lane & 7) * 4], page + g.scale_off + lane * 16);
+    dp_cp16(&st.mean[lane >> 3][(lane & 7) * 4], page + g.mean_off + lane * 16);
+    if (lane < 4) dp_cp16((uint8_t*)&st.hdr + lane * 16, page + g.hdr_off + lane * 16);
+    else dp_cp16(st.ovf + (lane - 4) * 4, page + g.hdr_off + TQ_OVF_OFF + (lane - 4) * 16);
+  };
+  auto copy_values = [&](const uint8_t* page) {
+    const uint8_t* src = page + g.v_off + (size_t)(t0 / TQ_GROUP_TOK) * VGB;
+#pragma unroll
+    for (int i = 0; i < 4 * VGB / 512; ++i)
+      dp_cp16(st.values + (32 * i + lane) * 16, src + (32 * i + lane) * 16);
+    if (lane < 16) dp_cp16(st.norms + lane * 4, page + g.norm_off + t0 * 4 + lane * 16);
+  };
+  static_assert(sizeof(PageHeader) == 64 && TQ_OVF_CAP * 4 == 28 * 16, "pieces of the tail");
+
+  // this lane's heads are 2 c and 2 c + 1, its channels 16 mt + r and 16 mt + r + 8
+  float acc[8][4], m_run[2], l_run[2];
+  auto reset = [&]() {
+#pragma unroll
+    for (int mt = 0; mt < 8; ++mt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[mt][i] = 0.0f;
+    m_run[0] = m_run[1] = -INFINITY;
+    l_run[0] = l_run[1] = 0.0f;
+  };
+  // the four warps' states become one partial
+  auto flush = [&](int unit, int gt, int slot) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) l_run[x] += __shfl_xor_sync(0xffffffffu, l_run[x], o);
+      if (r == 0) {
+        sh.m[gi][warp][2 * c + x] = m_run[x];
+        sh.l[gi][warp][2 * c + x] = l_run[x];
+      }
+    }
+    group_sync();  // (and every warp is done with its corrections: the sums take their place)
+    float f[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      float M = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) M = fmaxf(M, sh.m[gi][w][2 * c + x]);
+      f[x] = m_run[x] > -INFINITY ? __expf(m_run[x] - M) : 0.0f;
+    }
+    float* sums = &sh.corr[gi][0][0][0];  // [8 heads][128], bits 3 and 4 of the channel by the head
+    for (int w = 0; w < 4; ++w) {
+      if (warp == w) {
+#pragma unroll
+        for (int mt = 0; mt < 8; ++mt)
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              float* at = &sums[(2 * c + x) * TQ_D + ((16 * mt + 8 * y + r) ^ (8 * c))];
+              const float v = acc[mt][2 * y + x] * f[x];
+              *at = w == 0 ? v : *at + v;
+            }
+      }
+      group_sync();
+    }
+    float* pp = slot_of(unit, gt, slot);
+#pragma unroll
+    for (int gg = 0; gg < GT; ++gg)
+      if (gt * GT + gg < G) pp[gg * TQ_PART_STRIDE + 2 + gtid] = sums[gg * TQ_D + (gtid ^ (8 * (gg >> 1)))];
+    if (gtid < GT && gt * GT + gtid < G) {
+      float M = -INFINITY, L = 0.0f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) M = fmaxf(M, sh.m[gi][w][gtid]);
+#pragma unroll
+      for (int w = 0; w < 4; ++w)
+        L += sh.m[gi][w][gtid] > -INFINITY ? sh.l[gi][w][gtid] * __expf(sh.m[gi][w][gtid] - M) : 0.0f;
+      pp[gtid * TQ_PART_STRIDE] = M;
+      pp[gtid * TQ_PART_STRIDE + 1] = L;
     }
   };
 
-  const size_t out0 = ((size_t)unit * g.max_splits + split) * G + gt * GT;
-  if (cold) {
-    unsigned long long acc[8][NP];  // channels 64 (warp & 1) + 8 k + lane / 4
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-#pragma unroll
-      for (int x = 0; x < NP; ++x) acc[k][x] = 0ull;
-    const int b0 = min(a.block_begin, nb), b1 = a.block_end < 0 ? nb : min(a.block_end, nb);
-    const int nbr = max(b1 - b0, 0);
-    const int p_lo = b0 + (int)((long)nbr * split / a.ns_cold);
-    const int p_hi = b0 + (int)((long)nbr * (split + 1) / a.ns_cold);
-    const size_t u_idx = unit_index(g, a.layer, seq, head);
-    for (int pg = p_lo; pg < p_hi; ++pg) {
-      const uint8_t* page = a.pages + page_offset(g, a.layer, seq, head, pg);
-      // the two tokens' code rows, on their way while the weights are formed
-      uint4 row[2][4];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          row[h][v] = ((const uint4*)(page + (64 * warp + 32 * h + lane) * (TQ_D / 2)))[v];
-      {
-        const float sc = ((const float*)(page + g.scale_off))[tid];
-        const float mu = ((const float*)(page + g.mean_off))[tid];
-#pragma unroll
-        for (int gg = 0; gg < GT; ++gg) {
-          const float qv = q_s[tid][gg];
-          w_s[tid][gg] = qv * sc;
-          float b = qv * mu;
-#pragma unroll
-          for (int o = 16; o >= 1; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-          if (lane == 0) bias_w[warp][gg] = b;
-          s_s[gg][tid] = 0.0f;
-          s_s[gg][tid + 128] = 0.0f;
-        }
+  // (neighbouring shares go to different SMs: where there are few, each has one to itself)
+  const int me = gi * gridDim.x + blockIdx.x;
+  const long n_shares = a.ns_cold > 0 ? (total + share - 1) / share : 0;
+  for (long k = me; k < n_shares; k += n_groups) {
+    const long lo = k * share;
+    const int count = (int)min((long)share, total - lo);
+    Pos p;
+    {  // the sequence that holds page lo of the list: the last one that starts at or before it
+      int x = 0, y = n_seqs - 1;
+      while (x < y) {
+        const int mid = (x + y + 1) >> 1;
+        if ((long)sh.cum[mid] * rows_per_seq <= lo) x = mid;
+        else y = mid - 1;
       }
-      __syncthreads();
-      if (g.outlier_k > 0) {
-        // ordered by token, then channel: the thread with a token's first entry adds up all of
-        // them, so the sum does not depend on timing
-        const PageMeta pm = a.page_meta[u_idx * g.max_blocks + pg];
-        const uint32_t* ent = a.pool_dec + u_idx * (size_t)g.pool_entries + pm.off;
-        for (uint32_t e = tid; e < pm.cnt; e += DP_THREADS) {
-          const int tk = (int)(ent[e] >> 24);
-          if (e > 0 && (int)(ent[e - 1] >> 24) == tk) continue;
-          float sum[GT];
-#pragma unroll
-          for (int gg = 0; gg < GT; ++gg) sum[gg] = 0.0f;
-          for (uint32_t j = e; j < pm.cnt; ++j) {
-            const uint32_t wv = ent[j];
-            if ((int)(wv >> 24) != tk) break;
-            const float delta = __half2float(__ushort_as_half((unsigned short)(wv & 0xffff)));
-            const float* qr = q_s[(wv >> 16) & 127];
-#pragma unroll
-            for (int gg = 0; gg < GT; ++gg) sum[gg] += qr[gg] * delta;
-          }
-#pragma unroll
-          for (int gg = 0; gg < GT; ++gg) s_s[gg][tk] = sum[gg];
-        }
-      }
-      __syncthreads();
-      {
-        // eight channels at a time, then those sums: shorter chains of rounding than one of 128
-        unsigned long long dot[2][NP], sub[2][NP];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int x = 0; x < NP; ++x) dot[h][x] = sub[h][x] = 0ull;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const uint32_t cw[2][4] = {{row[0][v].x, row[0][v].y, row[0][v].z, row[0][v].w},
-                                     {row[1][v].x, row[1][v].y, row[1][v].z, row[1][v].w}};
-#pragma unroll
-          for (int n = 0; n < 32; ++n) {
-            unsigned long long w2[NP];
-#pragma unroll
-            for (int x = 0; x < NP; x += 2) {
-              const ulonglong2 t = *(const ulonglong2*)&w_s[32 * v + n][2 * x];
-              w2[x] = t.x;
-              w2[x + 1] = t.y;
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const float lv = nf4_s[(cw[h][n >> 3] >> (4 * (n & 7))) & 15];
-              const unsigned long long l2 = dp_pack(lv, lv);
-#pragma unroll
-              for (int x = 0; x < NP; ++x) {
-                sub[h][x] = (n & 7) == 0 ? dp_mul2(l2, w2[x]) : dp_fma2(l2, w2[x], sub[h][x]);
-                if ((n & 7) == 7) dot[h][x] = dp_add2(dot[h][x], sub[h][x]);
-              }
-            }
-          }
-          if (v == 1) {  // the first half of the channels joins the corrections
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int x = 0; x < NP; ++x) {
-                const float2 e = dp_unpack(dot[h][x]);
-                s_s[2 * x][64 * warp + 32 * h + lane] += e.x;
-                s_s[2 * x + 1][64 * warp + 32 * h + lane] += e.y;
-                dot[h][x] = 0ull;
-              }
-          }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int t = 64 * warp + 32 * h + lane;
-#pragma unroll
-          for (int x = 0; x < NP; ++x) {
-            const float2 e = dp_unpack(dot[h][x]);
-            const float d2[2] = {e.x, e.y};
-#pragma unroll
-            for (int y = 0; y < 2; ++y) {
-              const int gg = 2 * x + y;
-              const float bias = bias_w[0][gg] + bias_w[1][gg] + bias_w[2][gg] + bias_w[3][gg];
-              s_s[gg][t] = (d2[y] + bias + s_s[gg][t]) * a.scale;
-            }
-          }
-        }
-      }
-      __syncthreads();
-      const float* norms = (const float*)(page + g.norm_off);
-      softmax(DP_S, [&](int t) { return norms[t]; });
-      __syncthreads();
-      {
-        const int half = warp & 1;
-#pragma unroll
-        for (int x = 0; x < NP; ++x) {
-          const unsigned long long f2 = dp_pack(f_s[2 * x], f_s[2 * x + 1]);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) acc[k][x] = dp_mul2(acc[k][x], f2);
-        }
-        const int c4 = lane & 3;
-#pragma unroll 1
-        for (int gq = warp >> 1; gq < DP_S / TQ_GROUP_TOK; gq += 2) {
-          const uint8_t* grp = page + g.v_off + (size_t)gq * v_group_bytes(vb);
-          uint32_t rec[4];
-          if (vb == 4) {
-            const uint4 r = *(const uint4*)(grp + half * 512 + lane * 16);
-            rec[0] = r.x; rec[1] = r.y; rec[2] = r.z; rec[3] = r.w;
-          } else {
-            // bytes 12 half .. + 11 of the lane's 24-byte record (parts of 8 bytes)
-            const uint2 mid = *(const uint2*)(grp + 256 + lane * 8);
-            const uint2 end = *(const uint2*)(grp + half * 512 + lane * 8);
-            rec[0] = half ? mid.y : end.x;
-            rec[1] = half ? end.x : end.y;
-            rec[2] = half ? end.y : mid.x;
-            rec[3] = 0u;
-          }
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {  // tokens 2 c4, 2 c4 + 1 of the group's lower, upper eight
-            unsigned long long pr[2][NP];
-#pragma unroll
-            for (int o = 0; o < 2; ++o)
-#pragma unroll
-              for (int x = 0; x < NP; x += 2) {
-                const ulonglong2 t =
-                    *(const ulonglong2*)&p_s[16 * gq + 8 * hh + 2 * c4 + o][2 * x];
-                pr[o][x] = t.x;
-                pr[o][x + 1] = t.y;
-              }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const int p = 2 * k + hh;
-              uint32_t ca, cb;
-              if (vb == 4) {
-                const uint32_t b = rec[p >> 2] >> (8 * (p & 3));
-                ca = b & 15;
-                cb = (b >> 4) & 15;
-              } else {
-                const int bit = 6 * p;
-                const uint32_t b = __funnelshift_r(rec[bit >> 5], rec[(bit >> 5) + 1], bit & 31);
-                ca = b & 7;
-                cb = (b >> 3) & 7;
-              }
-              const float va = cent_s[ca], vc = cent_s[cb];
-              const unsigned long long a2 = dp_pack(va, va), c2 = dp_pack(vc, vc);
-#pragma unroll
-              for (int x = 0; x < NP; ++x)  // (two tokens, then the sum: half the chain)
-                acc[k][x] = dp_add2(acc[k][x], dp_fma2(c2, pr[1][x], dp_mul2(a2, pr[0][x])));
-            }
-          }
-        }
-      }
-      // (no barrier: what the next page writes first is not read by the value phase)
+      p.seq = x;
+      p.n = sh.cum[x + 1] - sh.cum[x];
+      const int rem = (int)(lo - (long)sh.cum[x] * rows_per_seq);
+      p.row = rem / p.n;
+      p.page = rem - p.row * p.n;
     }
-    // lanes of a quad hold different tokens of the same channels, and so do warps w and w + 2
-    __syncthreads();
-    float* mrg = &p_s[0][0];  // [GT][D]
-    static_assert(GT * TQ_D <= DP_S * PROW, "merge area");
-    for (int part = 0; part < 2; ++part) {
-      if (warp >> 1 == part) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-#pragma unroll
-          for (int x = 0; x < NP; ++x) {
-            const float2 v = dp_unpack(acc[k][x]);
-            float vv[2] = {v.x, v.y};
-#pragma unroll
-            for (int y = 0; y < 2; ++y) {
-              vv[y] += __shfl_xor_sync(0xffffffffu, vv[y], 1);
-              vv[y] += __shfl_xor_sync(0xffffffffu, vv[y], 2);
-              if ((lane & 3) == 0) {
-                float* dst = mrg + (2 * x + y) * TQ_D + 64 * (warp & 1) + 8 * k + (lane >> 2);
-                *dst = part == 0 ? vv[y] : *dst + vv[y];
-              }
-            }
-          }
-      }
-      __syncthreads();
+    {
+      const uint8_t* page = page_at(p);
+      copy_keys(page);
+      dp_commit();
+      copy_values(page);
+      dp_commit();
     }
+    bool fresh = true;  // the row's query has to be loaded
+    for (int i = 0; i < count; ++i) {
+      const int unit = (seq0 + p.seq) * H + p.row / tiles, gt = p.row % tiles;
+      if (fresh) {
+        group_sync();  // (the queries and sums of the row before are no longer read)
+        load_q(unit, gt);
+        reset();
+        group_sync();
+        fresh = false;
+      }
+      Pos next = p;
+      advance(next);
+      const uint8_t* next_page = i + 1 < count ? page_at(next) : nullptr;
+
+      asm volatile("cp.async.wait_group 1;" ::: "memory");  // the key half has landed
+      __syncwarp();
+      // weights: k-step j takes channels 32 c + 4 j .. + 3 of this lane, column r is head r
+      uint32_t bh[8][2], bl[8][2];
+      float bias2[2], inv2[2];
+      {
+        float w[8][4], mx = 0.0f;
+        float4 b4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int gg = 0; gg < GT; ++gg)
-      if (gt * GT + gg < G) a.partials[(out0 + gg) * TQ_PART_STRIDE + 2 + tid] = mrg[gg * TQ_D + tid];
-  } else {
-    unsigned long long acc[NP];  // channel tid
+        for (int j = 0; j < 8; ++j) {
+          const float4 s4 = *(const float4*)&st.scale[c][4 * j], m4 = *(const float4*)&st.mean[c][4 * j];
+          const int d = 32 * c + 4 * j;
+          const float q0 = q_s[q_row(d)][r], q1 = q_s[q_row(d + 1)][r], q2 = q_s[q_row(d + 2)][r],
+                      q3 = q_s[q_row(d + 3)][r];
+          w[j][0] = q0 * s4.x, w[j][1] = q1 * s4.y, w[j][2] = q2 * s4.z, w[j][3] = q3 * s4.w;
+          b4.x += q0 * m4.x, b4.y += q1 * m4.y, b4.z += q2 * m4.z, b4.w += q3 * m4.w;
 #pragma unroll
-    for (int x = 0; x < NP; ++x) acc[x] = 0ull;
-    const int j = split - a.ns_cold, dt = g.kv_dtype;
-    const int hot_start = nb * DP_S, hot_len = a.with_hot ? N - hot_start : 0;
+          for (int x = 0; x < 4; ++x) mx = fmaxf(mx, fabsf(w[j][x]));
+        }
+        float bias = (b4.x + b4.y) + (b4.z + b4.w);
+        bias += __shfl_xor_sync(0xffffffffu, bias, 1);
+        bias += __shfl_xor_sync(0xffffffffu, bias, 2);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float inv;
+        const float up = dp_lift(mx, 13, inv);
+        inv *= inv_k;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {  // of heads 2 c + x
+          bias2[x] = __shfl_sync(0xffffffffu, bias, 8 * c + 4 * x);
+          inv2[x] = __shfl_sync(0xffffffffu, inv, 8 * c + 4 * x);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dp_split(w[j][0] * up, w[j][1] * up, bh[j][0], bl[j][0]);
+          dp_split(w[j][2] * up, w[j][3] * up, bh[j][1], bl[j][1]);
+        }
+      }
+
+      float s[4][4];  // tile h: (token r, heads 2 c, 2 c + 1), (token r + 8, ...)
+      const bool spilled = (st.hdr.flags & TQ_PAGE_SPILLED) != 0;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        {  // outlier corrections of 32 tokens, a lane per token
+          const int tok = 32 * half + lane;  // of the strip
+          float e8[GT];
+#pragma unroll
+          for (int x = 0; x < GT; ++x) e8[x] = 0.0f;
+          auto add = [&](float delta, int row) {
+            const float4 qa = *(const float4*)&q_s[row][0], qb = *(const float4*)&q_s[row][4];
+            e8[0] += qa.x * delta, e8[1] += qa.y * delta, e8[2] += qa.z * delta, e8[3] += qa.w * delta;
+            e8[4] += qb.x * delta, e8[5] += qb.y * delta, e8[6] += qb.z * delta, e8[7] += qb.w * delta;
+          };
+          if (g.outlier_k > 0 && !spilled) {
+#pragma unroll
+            for (int j = 0; j < TQ_ELL_SLOTS; ++j)
+              add(__half2float(__ushort_as_half(st.delta[j][tok])), st.col[j][tok]);
+          }
+          __syncwarp();  // (the tiles of the half before have been read)
+          *(float4*)&corr[lane][0] = make_float4(e8[0], e8[1], e8[2], e8[3]);
+          *(float4*)&corr[lane][4] = make_float4(e8[4], e8[5], e8[6], e8[7]);
+          __syncwarp();
+          if (g.outlier_k > 0) {
+            // the rest of the list, ordered by token: the lane with a token's first entry adds up all of
+            // them, so the sum does not depend on timing
+            const uint32_t* list = st.ovf;
+            int e0 = st.hdr.ovf_start[warp], e1 = st.hdr.ovf_start[warp + 1];
+            if (spilled) {
+              const size_t slab = unit_index(g, a.layer, seq0 + p.seq, p.row / tiles) * (size_t)g.pool_entries;
+              list = a.pool_dec + slab + st.hdr.off;
+              e0 = 0, e1 = (int)st.hdr.cnt;
+            }
+            for (int e = e0 + lane; e < e1; e += 32) {
+              uint32_t v = list[e];
+              const int tk = (int)(v >> 24);
+              if (tk >> 5 != (t0 >> 5) + half || (e > e0 && (int)(list[e - 1] >> 24) == tk)) continue;
+#pragma unroll
+              for (int x = 0; x < GT; ++x) e8[x] = corr[tk & 31][x];
+              for (int j = e;;) {
+                add(__half2float(__ushort_as_half((unsigned short)(v & 0xffffu))),
+                    q_row((v >> 16) & 127));
+                if (++j >= e1) break;
+                v = list[j];
+                if ((int)(v >> 24) != tk) break;
+              }
+#pragma unroll
+              for (int x = 0; x < GT; ++x) corr[tk & 31][x] = e8[x];
+            }
+            __syncwarp();
+          }
+        }
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) {
+          const int h = 2 * half + h2;
+          uint32_t kw[2][4];
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const uint4 v = *(const uint4*)(st.keys + (16 * h + 8 * x + r) * (TQ_D / 2) + c * 16);
+            kw[x][0] = v.x, kw[x][1] = v.y, kw[x][2] = v.z, kw[x][3] = v.w;
+          }
+          float sum[2][4];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            uint32_t ah[4], al[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {  // tokens r, r + 8; bytes 2 j, 2 j + 1
+              const uint32_t b = __byte_perm(kw[x & 1][j >> 1], 0, 0x4440 + 2 * (j & 1) + (x >> 1));
+              const uint2 t = dp_lut(lutk + b * 128);
+              ah[x] = t.x, al[x] = t.y;
+            }
+            float d[4];
+            dp_product(d, ah, al, bh[j], bl[j]);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) sum[j & 1][x] = j < 2 ? d[x] : sum[j & 1][x] + d[x];
+          }
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const float2 e2 = *(const float2*)&corr[16 * h2 + 8 * x + r][2 * c];
+            s[h][2 * x] = (fmaf(sum[0][2 * x] + sum[1][2 * x], inv2[0], bias2[0]) + e2.x) * a.scale;
+            s[h][2 * x + 1] =
+                (fmaf(sum[0][2 * x + 1] + sum[1][2 * x + 1], inv2[1], bias2[1]) + e2.y) * a.scale;
+          }
+        }
+      }
+      __syncwarp();  // the key half has been read
+      if (next_page != nullptr) copy_keys(next_page);
+      dp_commit();
+      asm volatile("cp.async.wait_group 1;" ::: "memory");  // the value half has landed
+      __syncwarp();
+
+      // softmax over the strip; the largest norm sets the scale of the value operand
+      float nv[4][2], n_max = 0.0f;
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          nv[h][x] = st.norms[16 * h + 8 * x + r];
+          n_max = fmaxf(n_max, nv[h][x]);
+        }
+      float f[2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) mx = fmaxf(mx, fmaxf(s[h][x], s[h][2 + x]));
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float m_new = fmaxf(m_run[x], mx);
+        const bool any = m_new > -INFINITY;
+        f[x] = any ? __expf(m_run[x] - m_new) : 1.0f;
+        float sum = 0.0f;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            s[h][2 * y + x] = any ? __expf(s[h][2 * y + x] - m_new) : 0.0f;
+            sum += s[h][2 * y + x];
+          }
+        l_run[x] = l_run[x] * f[x] + sum;
+        m_run[x] = m_new;
+      }
+#pragma unroll
+      for (int mt = 0; mt < 8; ++mt) {
+        acc[mt][0] *= f[0], acc[mt][1] *= f[1];
+        acc[mt][2] *= f[0], acc[mt][3] *= f[1];
+      }
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1) n_max = fmaxf(n_max, __shfl_xor_sync(0xffffffffu, n_max, o));
+      float inv_n;
+      const float up_n = dp_lift(n_max, 13, inv_n);
+      inv_n *= inv_v;
+
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        uint32_t ph[2], pl[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {  // tokens 0-7, 8-15 of the tile
+          const float n = nv[h][x] * up_n;
+          uint32_t hi, lo2;
+          dp_split(s[h][2 * x] * n, s[h][2 * x + 1] * n, hi, lo2);
+          ph[x] = dp_transpose(hi);
+          pl[x] = dp_transpose(lo2);
+        }
+        const uint8_t* grp = st.values + h * VGB;
+        uint32_t rec[9];
+        if (VB == 4) {
+          const uint4 x = *(const uint4*)(grp + lane * 16), y = *(const uint4*)(grp + 512 + lane * 16);
+          rec[0] = x.x, rec[1] = x.y, rec[2] = x.z, rec[3] = x.w;
+          rec[4] = y.x, rec[5] = y.y, rec[6] = y.z, rec[7] = y.w;
+        } else {
+#pragma unroll
+          for (int x = 0; x < 3; ++x) {
+            const uint2 v = *(const uint2*)(grp + 256 * x + lane * 8);
+            rec[2 * x] = v.x, rec[2 * x + 1] = v.y;
+          }
+          rec[6] = 0u;
+        }
+#pragma unroll
+        for (int mt = 0; mt < 8; ++mt) {
+          uint32_t ah[4], al[4];
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            // channels r, r + 8; tokens 0-7, 8-15: pairs 4 mt, 4 mt + 2, 4 mt + 1, 4 mt + 3 of the record
+            const int pr = 4 * mt + 2 * (x & 1) + (x >> 1);
+            uint32_t at;
+            if (VB == 4) {
+              at = __byte_perm(rec[pr >> 2], 0, 0x4440 + (pr & 3)) * 128u;
+            } else {  // the 6-bit field at bit 6 pr, moved to bits 7 .. 12
+              const int bit = 6 * pr, wd = bit >> 5, b = bit & 31;
+              const uint32_t v = b < 7    ? rec[wd] << (7 - b)
+                                 : b > 26 ? __funnelshift_r(rec[wd], rec[wd + 1], b - 7)
+                                          : rec[wd] >> (b - 7);
+              at = v & 0x1f80u;
+            }
+            const uint2 t = dp_lut(lutv + at);
+            ah[x] = t.x, al[x] = t.y;
+          }
+          float d[4];
+          dp_product(d, ah, al, ph, pl);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) acc[mt][x] = fmaf(d[x], inv_n, acc[mt][x]);
+        }
+      }
+      __syncwarp();  // the value half has been read
+      if (next_page != nullptr) copy_values(next_page);
+      dp_commit();
+
+      if (next.page == 0 || i + 1 == count) {  // the share leaves the row, or ends
+        const long row0 = (long)sh.cum[p.seq] * rows_per_seq + (long)p.row * p.n;  // the row's first page
+        const int slot = (int)(k - row0 / share);
+        flush(unit, gt, slot);
+        if (next.page == 0) mark_empty(unit, gt, slot + 1, a.ns_cold);
+        fresh = true;
+      }
+      p = next;
+    }
+  }
+
+  // ---- the uncompressed window -------------------------------------------------------------------
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  DpHot& ht = sh.group[gi].hot;
+  const int dt = g.kv_dtype, esz = elem_size(dt), row_bytes = TQ_D * esz, row_step = row_bytes + 16;
+  // (the splits start with the groups that have the least of the pages)
+  for (int item = n_groups - 1 - me; item < n_seqs * rows_per_seq * a.ns_hot; item += n_groups) {
+    const int split = item % a.ns_hot, row = item / a.ns_hot % rows_per_seq;
+    const int seq = seq0 + item / a.ns_hot / rows_per_seq, head = row / tiles, gt = row % tiles;
+    const int unit = seq * H + head;
+    const int N = a.seq_len[a.layer * g.n_seqs + seq];
+    const int hot_start = n_cold_blocks(N, g.hot_window, DP_S) * DP_S;
+    const int hot_len = a.with_hot ? N - hot_start : 0;
     const int ng = (hot_len + TQ_GROUP_TOK - 1) / TQ_GROUP_TOK;
-    const int t_lo = (int)((long)ng * j / a.ns_hot) * TQ_GROUP_TOK;
-    const int t_hi = min((int)((long)ng * (j + 1) / a.ns_hot) * TQ_GROUP_TOK, hot_len);
-    const size_t ring = hot_offset_elems(g, a.layer, seq, head);
-    for (int t0 = t_lo; t0 < t_hi; t0 += DP_HOT) {
-      const int n_tok = min(DP_HOT, t_hi - t0);
-      if (tid < n_tok) {
-        const size_t at = ring + (size_t)((hot_start + t0 + tid) % g.hot_cap) * TQ_D;
-        unsigned long long dot[NP], sub[NP], low[NP];
+    const int t_lo = (int)((long)ng * split / a.ns_hot) * TQ_GROUP_TOK;
+    const int t_hi = min((int)((long)ng * (split + 1) / a.ns_hot) * TQ_GROUP_TOK, hot_len);
+    if (t_lo >= t_hi) {
+      mark_empty(unit, gt, a.ns_cold + split, a.ns_cold + split + 1);
+      continue;
+    }
+    const size_t ring = hot_offset_elems(g, a.layer, seq, head) * esz;
+    const int slot0 = (hot_start + t_lo) % g.hot_cap;
+    // rows [t, t + n) of a ring into shared memory
+    auto copy_rows = [&](const void* from, int t, int n) {
+      const int pieces = row_bytes / 16;
+      for (int i = gtid; i < n * pieces; i += DP_GTH) {
+        const int x = i / pieces, pc = i - x * pieces;
+        int slot = slot0 + (t - t_lo) + x;
+        while (slot >= g.hot_cap) slot -= g.hot_cap;
+        dp_cp16(ht.rows + x * row_step + pc * 16, (const uint8_t*)from + ring + (size_t)slot * row_bytes + pc * 16);
+      }
+    };
+    group_sync();  // (what the group did before in this memory is over)
+    copy_rows(a.hot_k, t_lo, min(DP_HOT, t_hi - t_lo));
+    load_q(unit, gt);
+    float m_h[2], l_h[2];  // of heads 2 warp + i, the same in every lane
+    unsigned long long av[NP];  // channel gtid
 #pragma unroll
-        for (int x = 0; x < NP; ++x) dot[x] = sub[x] = low[x] = 0ull;
+    for (int i = 0; i < 2; ++i) {
+      m_h[i] = -INFINITY;
+      l_h[i] = 0.0f;
+    }
+#pragma unroll
+    for (int x = 0; x < NP; ++x) av[x] = 0ull;
+    for (int t = t_lo; t < t_hi; t += DP_HOT) {
+      const int n_tok = min(DP_HOT, t_hi - t);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      group_sync();
+      {  // scores: thread (token, four heads)
+        const int tok = gtid & (DP_HOT - 1), h4 = gtid / DP_HOT * 4;
+        if (tok < n_tok) {
+          const uint8_t* kr = ht.rows + tok * row_step;
+          unsigned long long dot[2] = {0ull, 0ull}, low[2] = {0ull, 0ull}, sub[2];
 #pragma unroll 2
-        for (int d0 = 0; d0 < TQ_D; d0 += 8) {
-          float kv[8];
-          if (dt == TQ_F32) {
-            const float4 x = *(const float4*)((const float*)a.hot_k + at + d0);
-            const float4 y = *(const float4*)((const float*)a.hot_k + at + d0 + 4);
-            kv[0] = x.x; kv[1] = x.y; kv[2] = x.z; kv[3] = x.w;
-            kv[4] = y.x; kv[5] = y.y; kv[6] = y.z; kv[7] = y.w;
-          } else {
-            const uint4 x = *(const uint4*)((const uint16_t*)a.hot_k + at + d0);
-            const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+          for (int d0 = 0; d0 < TQ_D; d0 += 8) {
+            float kv[8];
+            if (dt == TQ_F32) {
+              const float4 x = *(const float4*)(kr + 4 * d0), y = *(const float4*)(kr + 4 * d0 + 16);
+              kv[0] = x.x; kv[1] = x.y; kv[2] = x.z; kv[3] = x.w;
+              kv[4] = y.x; kv[5] = y.y; kv[6] = y.z; kv[7] = y.w;
+            } else {
+              const uint4 x = *(const uint4*)(kr + 2 * d0);
+              const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (dt == TQ_F16) {
-                const float2 f = __half22float2(*(const __half2*)&w[i]);
-                kv[2 * i] = f.x; kv[2 * i + 1] = f.y;
-              } else {
-                kv[2 * i] = __uint_as_float(w[i] << 16);
-                kv[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+              for (int i = 0; i < 4; ++i) {
+                if (dt == TQ_F16) {
+                  const float2 e = __half22float2(*(const __half2*)&w[i]);
+                  kv[2 * i] = e.x; kv[2 * i + 1] = e.y;
+                } else {
+                  kv[2 * i] = __uint_as_float(w[i] << 16);
+                  kv[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                }
               }
             }
-          }
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const unsigned long long k2 = dp_pack(kv[i], kv[i]);
+            for (int i = 0; i < 8; ++i) {
+              const unsigned long long k2 = dp_pack(kv[i], kv[i]);
+              const ulonglong2 qv = *(const ulonglong2*)&q_s[q_row(d0 + i)][h4];
+              sub[0] = i == 0 ? dp_mul2(k2, qv.x) : dp_fma2(k2, qv.x, sub[0]);
+              sub[1] = i == 0 ? dp_mul2(k2, qv.y) : dp_fma2(k2, qv.y, sub[1]);
+            }
 #pragma unroll
-            for (int x = 0; x < NP; x += 2) {
-              const ulonglong2 t = *(const ulonglong2*)&q_s[d0 + i][2 * x];
-              sub[x] = i == 0 ? dp_mul2(k2, t.x) : dp_fma2(k2, t.x, sub[x]);
-              sub[x + 1] = i == 0 ? dp_mul2(k2, t.y) : dp_fma2(k2, t.y, sub[x + 1]);
+            for (int x = 0; x < 2; ++x) {
+              if (d0 == TQ_D / 2) {  // (the halves add up separately)
+                low[x] = dot[x];
+                dot[x] = 0ull;
+              }
+              dot[x] = dp_add2(dot[x], sub[x]);
             }
           }
 #pragma unroll
-          for (int x = 0; x < NP; ++x) {
-            if (d0 == TQ_D / 2) {  // (the halves add up separately)
-              low[x] = dot[x];
-              dot[x] = 0ull;
-            }
-            dot[x] = dp_add2(dot[x], sub[x]);
+          for (int x = 0; x < 2; ++x) {
+            const float2 e = dp_unpack(dp_add2(low[x], dot[x]));
+            ht.s[h4 + 2 * x][tok] = e.x * a.scale;
+            ht.s[h4 + 2 * x + 1][tok] = e.y * a.scale;
           }
-        }
-#pragma unroll
-        for (int x = 0; x < NP; ++x) {
-          const float2 e = dp_unpack(dp_add2(low[x], dot[x]));
-          s_s[2 * x][tid] = e.x * a.scale;
-          s_s[2 * x + 1][tid] = e.y * a.scale;
         }
       }
-      __syncthreads();
-      softmax(n_tok, [](int) { return 1.0f; });
-      __syncthreads();
+      group_sync();
+      copy_rows(a.hot_v, t, n_tok);  // (over the keys)
 #pragma unroll
-      for (int x = 0; x < NP; ++x) acc[x] = dp_mul2(acc[x], dp_pack(f_s[2 * x], f_s[2 * x + 1]));
-      int slot = (hot_start + t0) % g.hot_cap;
+      for (int i = 0; i < 2; ++i) {  // softmax: a warp takes two heads
+        const int gg = warp * 2 + i;
+        float sc[2], mx = -INFINITY;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          sc[x] = lane + 32 * x < n_tok ? ht.s[gg][lane + 32 * x] : -INFINITY;
+          mx = fmaxf(mx, sc[x]);
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float m_new = fmaxf(m_h[i], mx);
+        const bool any = m_new > -INFINITY;
+        const float fo = any ? __expf(m_h[i] - m_new) : 1.0f;
+        float sum = 0.0f;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float pv = any && lane + 32 * x < n_tok ? __expf(sc[x] - m_new) : 0.0f;
+          sum += pv;
+          ht.p[lane + 32 * x][gg] = pv;
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        l_h[i] = l_h[i] * fo + sum;
+        m_h[i] = m_new;
+        if (lane == 0) sh.f[gi][gg] = fo;
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      group_sync();
+#pragma unroll
+      for (int x = 0; x < NP; ++x)
+        av[x] = dp_mul2(av[x], dp_pack(sh.f[gi][2 * x], sh.f[gi][2 * x + 1]));
       for (int tb = 0; tb < n_tok; tb += 8) {  // eight tokens, then their sum
         unsigned long long sub[NP];
 #pragma unroll
         for (int x = 0; x < NP; ++x) sub[x] = 0ull;
-        const int m = min(8, n_tok - tb);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          if (t < m) {
-            const float v = dp_ld(a.hot_v, ring + (size_t)slot * TQ_D + tid, dt);
-            if (++slot == g.hot_cap) slot = 0;
+        for (int y = 0; y < 8; ++y) {
+          if (tb + y < n_tok) {
+            const float v = dp_ld(ht.rows + (tb + y) * row_step, gtid, dt);
             const unsigned long long v2 = dp_pack(v, v);
 #pragma unroll
             for (int x = 0; x < NP; x += 2) {
-              const ulonglong2 p = *(const ulonglong2*)&p_s[tb + t][2 * x];
-              sub[x] = dp_fma2(v2, p.x, sub[x]);
-              sub[x + 1] = dp_fma2(v2, p.y, sub[x + 1]);
+              const ulonglong2 pv = *(const ulonglong2*)&ht.p[tb + y][2 * x];
+              sub[x] = dp_fma2(v2, pv.x, sub[x]);
+              sub[x + 1] = dp_fma2(v2, pv.y, sub[x + 1]);
             }
           }
         }
 #pragma unroll
-        for (int x = 0; x < NP; ++x) acc[x] = dp_add2(acc[x], sub[x]);
+        for (int x = 0; x < NP; ++x) av[x] = dp_add2(av[x], sub[x]);
       }
-      // (no barrier: the next round's scores are not read here, its probabilities come after two)
+      group_sync();  // the rows, probabilities and factors have been read
+      if (t + DP_HOT < t_hi) copy_rows(a.hot_k, t + DP_HOT, min(DP_HOT, t_hi - t - DP_HOT));
     }
+    float* pp = slot_of(unit, gt, a.ns_cold + split);
 #pragma unroll
     for (int x = 0; x < NP; ++x) {
-      const float2 v = dp_unpack(acc[x]);
-      if (gt * GT + 2 * x < G) a.partials[(out0 + 2 * x) * TQ_PART_STRIDE + 2 + tid] = v.x;
-      if (gt * GT + 2 * x + 1 < G) a.partials[(out0 + 2 * x + 1) * TQ_PART_STRIDE + 2 + tid] = v.y;
+      const float2 v = dp_unpack(av[x]);
+      if (gt * GT + 2 * x < G) pp[(2 * x) * TQ_PART_STRIDE + 2 + gtid] = v.x;
+      if (gt * GT + 2 * x + 1 < G) pp[(2 * x + 1) * TQ_PART_STRIDE + 2 + gtid] = v.y;
     }
-  }
-  if (lane == 0) {
+    if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < HW; ++i) {
-      const int gg = warp * HW + i;
-      if (gt * GT + gg < G) {
-        a.partials[(out0 + gg) * TQ_PART_STRIDE] = m_run[i];
-        a.partials[(out0 + gg) * TQ_PART_STRIDE + 1] = l_run[i];
-      }
+      for (int i = 0; i < 2; ++i)
+        if (gt * GT + warp * 2 + i < G) {
+          pp[(warp * 2 + i) * TQ_PART_STRIDE] = m_h[i];
+          pp[(warp * 2 + i) * TQ_PART_STRIDE + 1] = l_h[i];
+        }
     }
   }
 }
 
+template <int VB>
+int launch_pages(const DecodeArgs& a, int ctas, cudaStream_t st) {
+  static_assert(sizeof(DpShared<VB>) <= 227 * 1024, "shared memory of one CTA");
+  int device = 0;
+  TQ_CUDA(cudaGetDevice(&device));
+  static bool attr_set[16] = {};  // per device: the attribute belongs to the device's context
+  if (!attr_set[device & 15]) {
+    TQ_CUDA(cudaFuncSetAttribute(decode_pages_kernel<VB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(DpShared<VB>)));
+    attr_set[device & 15] = true;
+  }
+  for (int s0 = 0; s0 < a.g.n_seqs; s0 += DP_SEQS)
+    decode_pages_kernel<VB><<<ctas, DP_THREADS, sizeof(DpShared<VB>), st>>>(
+        a, s0, a.g.n_seqs - s0 < DP_SEQS ? a.g.n_seqs - s0 : DP_SEQS);
+  return TQ_OK;
+}
+
 }  // namespace
 
-void tq_launch_decode_pages(const DecodeArgs& a, int n_units, cudaStream_t st) {
-  // Tiles of eight heads; a group of five to seven leaves up to three idle, one of nine to fifteen
-  // up to seven of its second tile.  Microseconds a layer, general kernel / this one (K4/V3, bf16; 64
-  // units of 700 to 12 000 tokens, 64 of 6 000, 8 of 32 768, 32 of 900):
-  //   5 heads   252 / 203   264 / 192   191 / 110   39 / 31
-  //   7 heads   254 / 203   266 / 192   192 / 110   39 / 31
-  //   8 heads   310 / 203   311 / 193   232 / 110   52 / 31   (where the general kernel is asked for)
-  //   9 heads   553 / 256   557 / 256   382 / 170   70 / 36
-  //  16 heads   552 / 257   555 / 256   379 / 170   74 / 36
-  const dim3 grid(a.ns_cold + a.ns_hot, n_units, (a.g.group + DP_GT - 1) / DP_GT);
-  decode_pages_kernel<<<grid, DP_THREADS, 0, st>>>(a);
+// Tiles of eight heads; a group of five to seven leaves up to three idle, one of nine to fifteen up to
+// seven of its second tile.  Microseconds of a decode call, general kernel / this one, merge included
+// (K4/V3, bf16; 64 units of 700 to 12 000 tokens, 64 of 6 000, 8 of 32 768, 32 of 900, 4 of 600):
+//   5 heads   258 / 78   269 / 68   199 / 55   44 / 23   40 / 21
+//   7 heads   260 / 80   271 / 71   200 / 54   44 / 23   40 / 21
+//   9 heads   558 / 126  562 / 114  390 / 77   75 / 32   65 / 21
+//  16 heads   557 / 134  560 / 113  387 / 81   79 / 33   66 / 21
+// What bounds it: the look-ups (shared memory) and the issue slots of the splits and products.
+int tq_launch_decode_pages(const DecodeArgs& a, int sm_count, cudaStream_t st) {
+  return a.g.value_bits == 3 ? launch_pages<3>(a, sm_count, st) : launch_pages<4>(a, sm_count, st);
 }
