@@ -1573,7 +1573,7 @@ int launch_encode_t(const EncodeArgs& a, const ValueTable& vt, int sm_count, int
     }
     const int ctas5 = (int)std::min<long>((total + ENC5_PARTS - 1) / ENC5_PARTS, (long)sm_count);
     auto values = [&](const EncodeArgs& av) {
-      if (tiles) return tq_launch_encode_values_tiles(av, vt, sm_count, device, st);
+      if (tiles) return tq_launch_encode_values_tiles(av, vt, tq_keys_block_form(g), sm_count, device, st);
       if (tc5 && g.value_bits == 3)
         encode_values_tc5_kernel<DT, 3><<<ctas5, ENC5_PARTS * TQ_D, ENC5_SMEM, st>>>(av);
       else if (tc5)

@@ -92,8 +92,9 @@ int tq_launch_encode_keys_block(const EncodeArgs& a, int device, cudaStream_t st
 
 // Value encoder for blocks of 128 or 256 tokens (encode_values.cu).
 constexpr float VALUE_SPAN = 1023.0f / 1024.0f;  // z = 1 still has a mantissa below 2^23
-int tq_launch_encode_values_tiles(const EncodeArgs& a, const ValueTable& vt, int sm_count, int device,
-                                  cudaStream_t st);
+// `after_keys`: the kernel before it in the stream is the key encoder of the same call.
+int tq_launch_encode_values_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys,
+                                  int sm_count, int device, cudaStream_t st);
 
 TQ_DEV uint32_t enc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // Shared-memory operand of tcgen05.mma, K-major without swizzling: 8 x 8 core matrices of 16-bit

@@ -122,6 +122,8 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   const int seq = a.seq_begin + blockIdx.z, head = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int p = tid & 63, seg = tid >> 6;  // channels 2p, 2p + 1; tokens seg * NT ...
+  // (the value encoder behind this kernel in the stream touches nothing that it writes)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int n0 = a.seq_len[a.layer * g.n_seqs + seq];
   const int nb0 = n_cold_blocks(n0, g.hot_window, EK_S);
   const int nb1 = n_cold_blocks(n0 + a.n_tokens, g.hot_window, EK_S);
