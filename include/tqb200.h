@@ -436,6 +436,18 @@ int32_t tq_profile_enable(tq_ctx* ctx, int32_t on);
  * combine-kernel milliseconds and the number of tq_decode calls they cover; resets. */
 int32_t tq_profile_read(tq_ctx* ctx, double* attn_ms, double* combine_ms, int32_t* n_calls);
 
+/* The bytes np.savez writes for `n` arrays (the container of a stored block, vllm_v1.py:113-196), on the
+ * host.  `parts` holds four words per member: bytes of its file name, bytes of its .npy header, address
+ * and bytes of its data; `text` holds name and header of each member, one after the other.  Returns
+ * the bytes written, -1 where they are not `out_bytes` (30 + 20 + 46 + twice the name, the header and the
+ * data per member, and 22) or exceed 31 bits. */
+int64_t tq_npz_write(int32_t n, const int64_t* parts, const char* text, void* out, int64_t out_bytes);
+
+/* Checks such an archive (records, checksums, .npy magic) and gives six words per member: offset and bytes
+ * of its file name, of its .npy header and of its data.  Returns the number of members; -1 for
+ * any other or damaged archive, or for more than `max_members`. */
+int32_t tq_npz_read(const void* blob, int64_t bytes, int32_t max_members, int64_t* members);
+
 #ifdef __cplusplus
 }
 #endif

@@ -126,6 +126,8 @@ SIGNATURES = {
     "tq_set_key_bias_means": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "tq_debug_trace": (C.c_int32, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]),
     "tq_profile_enable": (C.c_int32, [C.c_void_p, C.c_int32]),
+    "tq_npz_write": (C.c_int64, [C.c_int32, C.c_void_p, C.c_char_p, C.c_void_p, C.c_int64]),
+    "tq_npz_read": (C.c_int32, [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p]),
     "tq_profile_read": (C.c_int32, [C.c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_double),
                                     C.POINTER(C.c_int32)]),
 }

@@ -598,11 +598,11 @@ class KVContext:
         stores no means, so ``bias_means`` ``(n_kv_heads, D)`` of this block must be given."""
         self.import_block(layer, seq, block, self._from_blob(blob, bias_means))
 
-    def _from_blob(self, blob: bytes, bias_means) -> dict:
-        from .kv_blob import blob_to_block, block_from_parsed
+    def _from_blob(self, blob: bytes, bias_means, copy: bool = True) -> dict:
+        from .kv_blob import _parse, block_from_parsed
 
         return block_from_parsed(
-            blob_to_block(blob), key_mode=self.key_mode, mean_mask=self.key_mean_mask,
+            _parse(blob, copy=copy), key_mode=self.key_mode, mean_mask=self.key_mean_mask,
             bias_means=bias_means,
             geom=(self.geom.n_kv_heads, self.geom.block_tokens, self.geom.head_dim,
                   self.geom.value_bits))
@@ -650,7 +650,7 @@ class KVContext:
         self.clear(layer, seq)
         for b0 in range(0, len(state["blocks"]), _WIRE_CHUNK):
             self._import_blocks(layer, seq, b0, [
-                self._from_blob(blob, None if bias_means is None else bias_means[b0 + i])
+                self._from_blob(blob, None if bias_means is None else bias_means[b0 + i], copy=False)
                 for i, blob in enumerate(state["blocks"][b0:b0 + _WIRE_CHUNK])])
         if n:
             hot = [torch.from_numpy(np.ascontiguousarray(state[name])).view(self.kv_dtype)

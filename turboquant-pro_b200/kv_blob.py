@@ -15,6 +15,7 @@ takes, so a stored block goes into device pages without passing through dense te
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import functools
 import io
 import json
@@ -29,6 +30,11 @@ CODEC = "tqp-kv-npz/1"
 _OK_DTYPES = {"uint8", "int8", "int16", "int32", "int64", "float16", "float32", "float64", "bool"}
 
 __all__ = ["CODEC", "block_to_blob", "blob_to_block", "block_from_parsed"]
+
+
+@functools.lru_cache(maxsize=64)
+def _allowed(dtype) -> bool:
+    return str(dtype) in _OK_DTYPES
 
 
 def _tuple(v):
@@ -100,12 +106,14 @@ def block_to_blob(block: dict, *, key_mode: str = "nf4_asym", zero_point: str = 
 # ---- the archive ---------------------------------------------------------------------------
 # A blob is what np.savez writes: a zip archive of stored (uncompressed) .npy members.  zipfile and
 # the .npy header parser spend several times longer on the nine small headers of a block than the
-# checksums and copies of its 280 KB take, so the plain form is written and read here by the record
-# layouts of the zip format (PKWARE's APPNOTE, 4.3); everything else is left to numpy.
+# checksums and copies of its 280 KB take, so the plain form is written and read by the record
+# layouts of the zip format (PKWARE's APPNOTE, 4.3): by the library's csrc/archive.cu, in Python
+# where the library has not been built.  Everything else is left to numpy.
 _LOCAL = struct.Struct("<4s5H3L2H")       # local file header
 _CENTRAL = struct.Struct("<4s6H3L5H2L")   # central directory entry
 _END = struct.Struct("<4s4H2LH")          # end of central directory
 _ZIP64 = struct.Struct("<2H2Q")           # extra field with 64-bit sizes
+_MEMBERS = 64                             # most members the library is asked for
 _NPY = re.compile(rb"\{'descr': '([<|][a-z][0-9]+)', 'fortran_order': False, "
                   rb"'shape': \(((?:[0-9]+,(?: [0-9]+,)*(?: [0-9]+)?)?)\), \} *\n")
 
@@ -118,6 +126,74 @@ def _npy_header(descr: str, shape: tuple) -> bytes:
     return buf.getvalue()
 
 
+@functools.lru_cache(maxsize=256)
+def _npy_parse(head: bytes):
+    """Element type and shape a .npy header (magic and length included) gives, ``None`` for another
+    form than the plain one."""
+    head = _NPY.fullmatch(head[10:])
+    if head is None:
+        return None
+    shape = tuple(int(x) for x in head[2].split(b",") if x.strip())
+    try:
+        dtype = np.dtype(head[1].decode())
+    except TypeError:
+        return None
+    return None if dtype.hasobject else (dtype, shape)
+
+
+@functools.lru_cache(maxsize=1)
+def _native():
+    """The built library, ``None`` where there is none."""
+    from . import _lib
+
+    try:
+        return _lib.load()
+    except (RuntimeError, OSError, AttributeError):
+        return None
+
+
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = ctypes.py_object, [ctypes.c_void_p, ctypes.c_ssize_t]
+
+
+def _address(a) -> int:
+    return a.__array_interface__["data"][0]
+
+
+def _write_native(lib, arrays: dict) -> bytes:
+    text, parts, size = [], [], _END.size
+    for name, a in arrays.items():
+        file, head = (name + ".npy").encode("ascii"), _npy_header(a.dtype.str, a.shape)
+        text += [file, head]
+        parts += [len(file), len(head), _address(a), a.nbytes]
+        size += _LOCAL.size + _ZIP64.size + _CENTRAL.size + 2 * len(file) + len(head) + a.nbytes
+    out = _new_bytes(None, size)  # (filled before anyone else sees it)
+    if lib.tq_npz_write(len(arrays), (ctypes.c_int64 * len(parts))(*parts), b"".join(text),
+                        ctypes.cast(ctypes.c_char_p(out), ctypes.c_void_p), size) != size:
+        raise RuntimeError("the archive could not be written")
+    return out
+
+
+def _read_native(lib, blob, max_bytes: int, copy: bool):
+    raw = np.frombuffer(blob, dtype=np.uint8)
+    table = (ctypes.c_int64 * (6 * _MEMBERS))()
+    view, members, used = memoryview(raw), {}, 0
+    for i in range(lib.tq_npz_read(_address(raw), raw.size, _MEMBERS, table)):
+        name_at, n_name, head_at, n_head, at, n = table[6 * i:6 * i + 6]
+        file = bytes(view[name_at:name_at + n_name])
+        form = _npy_parse(bytes(view[head_at:head_at + n_head]))
+        used += n_head + n
+        if form is None or not file.isascii() or not file.endswith(b".npy") or used > max_bytes \
+                or form[0].itemsize * math.prod(form[1]) != n:
+            return None
+        name = file[:-4].decode()
+        if name in members:
+            return None
+        a = raw[at:at + n].view(form[0]).reshape(form[1])
+        members[name] = a if form[0] == np.uint8 and not copy else a.copy()
+    return members or None
+
+
 def _write_npz(arrays: dict) -> bytes:
     """The bytes np.savez writes for these arrays."""
     if any(a.dtype.hasobject or not a.flags.c_contiguous for a in arrays.values()) \
@@ -125,6 +201,8 @@ def _write_npz(arrays: dict) -> bytes:
         buf = io.BytesIO()
         np.savez(buf, **arrays)
         return buf.getvalue()
+    if (lib := _native()) is not None:
+        return _write_native(lib, arrays)
     out, central, at = [], [], 0
     for name, a in arrays.items():
         file = (name + ".npy").encode("ascii")
@@ -144,11 +222,14 @@ def _write_npz(arrays: dict) -> bytes:
     return b"".join(out + central + [end])
 
 
-def _read_npz(blob: bytes, max_bytes: int):
+def _read_npz(blob: bytes, max_bytes: int, copy: bool = True):
     """The members of an archive of the plain form above, ``{name: array}``; ``None`` for any other
-    one (and for one that is damaged): numpy then reads it, or says what is wrong."""
+    one (and for one that is damaged): numpy then reads it, or says what is wrong.  Without ``copy``
+    the members of bytes may be views of the blob."""
     if len(blob) < _END.size:
         return None
+    if (lib := _native()) is not None:
+        return _read_native(lib, blob, max_bytes, copy)
     end = len(blob) - _END.size
     sig, disk, disk_c, here, total, n_central, first, comment = _END.unpack_from(blob, end)
     if sig != b"PK\5\6" or disk or disk_c or here != total or comment or first + n_central != end:
@@ -177,16 +258,10 @@ def _read_npz(blob: bytes, max_bytes: int):
         n_head = int.from_bytes(data[8:10], "little")
         if bytes(data[:8]) != b"\x93NUMPY\x01\x00" or 10 + n_head > size or zlib.crc32(data) != crc:
             return None
-        head = _NPY.fullmatch(bytes(data[10:10 + n_head]))
-        if head is None:
+        form = _npy_parse(bytes(data[:10 + n_head]))
+        if form is None or form[0].itemsize * math.prod(form[1]) != size - 10 - n_head:
             return None
-        shape = tuple(int(x) for x in head[2].split(b",") if x.strip())
-        try:
-            dtype = np.dtype(head[1].decode())
-        except TypeError:
-            return None
-        if dtype.hasobject or dtype.itemsize * math.prod(shape) != size - 10 - n_head:
-            return None
+        dtype, shape = form
         name = file[:-4].decode()
         used += size
         if name in members or used > max_bytes:
@@ -214,9 +289,13 @@ def blob_to_block(blob: bytes, max_bytes: int = 1 << 30) -> dict:
     codec string other than ``tqp-kv-npz/1`` and for array dtypes outside the numeric
     whitelist (object arrays cannot be loaded at all: ``allow_pickle=False``).
     """
+    return _parse(blob, max_bytes)
+
+
+def _parse(blob: bytes, max_bytes: int = 1 << 30, copy: bool = True) -> dict:
     if len(blob) > max_bytes:
         raise ValueError(f"blob exceeds max_bytes ({len(blob)} > {max_bytes})")
-    members = _read_npz(blob, max_bytes)
+    members = _read_npz(blob, max_bytes, copy)
     with contextlib.nullcontext(members) if members is not None else \
             np.load(io.BytesIO(blob), allow_pickle=False) as z:
         names = list(z) if members is not None else z.files
@@ -232,7 +311,7 @@ def blob_to_block(blob: bytes, max_bytes: int = 1 << 30) -> dict:
             if name == "__header__":
                 continue
             a = z[name]
-            if str(a.dtype) not in _OK_DTYPES:
+            if not _allowed(a.dtype):
                 raise ValueError(f"dtype {a.dtype} of {name} is not allowed")
             total += a.nbytes
             if total > max_bytes:
