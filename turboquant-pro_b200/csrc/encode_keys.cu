@@ -15,11 +15,12 @@
 //   - outliers: where a block is cut into 32 groups of eight tokens, the k largest magnitudes of a
 //     channel lie in the k groups with the largest maxima (in a few more where maxima are equal),
 //     so only those groups are searched for the k-th magnitude and for the tokens that reach it.
-// Measured (B200): 8 x 16 384 fp16 tokens x 8 heads about 780 us with the general encoder, 248 us
-// here; 4001 float32 tokens x 32 heads about 300 us and 62 us; the 32 blocks of one flush, alone on the
-// GPU, 16 us.  Counters: 54 % of the issue slots with 16-bit tokens (two CTAs an SM; warps wait for
-// fixed latencies, then for barriers), 39 % with float32 (one CTA an SM, nothing to cover its
-// barriers and its load); DRAM at 17 %.
+// Measured (B200): 8 x 16 384 fp16 tokens x 8 heads about 780 us with the general encoder, 234 us
+// here; 4001 float32 tokens x 32 heads about 300 us and 60 us; the 32 blocks of one flush, alone on the
+// GPU, 16 us.  What bounds it: latency.  Cycles of a CTA with another beside it on the SM (fp16): first rows
+// 5.1 k, pass 1 4.5 k, table 3.5 k, pass 2 5.3 k, redos 1.5 k, outliers' search 5.4 k, their lists 6.7 k.
+// (With the table behind a barrier of its own, all rows waited for at once and the outliers' slots stored
+// one by one from the registers 246 us; with 512 threads a CTA 258 us.)
 // The passes read the block from shared memory, eight tokens an iteration: all loads of an
 // iteration first and its stores last, so that the eight chains of dependent steps overlap.
 #include "encode.cuh"
@@ -52,14 +53,16 @@ struct Ek {
   static constexpr int THREADS = 64 * SEG;
   // shared memory
   static constexpr int ROWS = EK_S * TQ_D * (DT == TQ_F32 ? 4 : 2);
-  static constexpr int TAB = EK_BINS * TQ_D * 4;       // group maxima, then the table, then the outlier list
-  static constexpr int IMG = EK_S * TQ_D / 2;          // the page's code rows
-  static constexpr int MM = 2 * SEG * TQ_D * 4;        // extremes of the segments, then the list of redos
+  static constexpr int TAB = EK_BINS * TQ_D * 4;       // the table, then the outlier list
+  static constexpr int IMG = EK_S * TQ_D / 2;          // group maxima, then the page's code rows
+  static constexpr int MM = 2 * SEG * TQ_D * 4;        // extremes of the segments, list of redos, the page's tail
   static constexpr int MASK = EK_S * 16;               // outlier channels of every token
   static constexpr int SMEM = ROWS + TAB + IMG + MM + MASK;
 };
 constexpr int EK_REDOS = EK_S / 8 * (TQ_D / 2);  // eight tokens of a channel pair each
-static_assert(EK_GROUPS * TQ_D * 4 <= Ek<TQ_F32>::TAB && EK_REDOS * 2 <= Ek<TQ_F16>::MM, "shared areas");
+static_assert(EK_GROUPS * TQ_D * 4 <= Ek<TQ_F32>::IMG && EK_REDOS * 2 <= Ek<TQ_F16>::MM &&
+                  TQ_TAIL_BYTES <= Ek<TQ_F16>::MM,
+              "shared areas");
 
 // column of channel ch in the table: a warp's 32 even (odd) channels on 32 different banks
 TQ_DEV int ek_col(int ch) { return (ch >> 1) + 64 * (ch & 1); }
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   __shared__ uint32_t s_off_pool, s_scan[EK_S / 32];
   __shared__ unsigned short s_row[EK_S], s_orow[EK_S];  // a token's first outlier, first overflow entry
   __shared__ int s_wide[TQ_WIDE];
-  __shared__ __align__(8) unsigned long long s_bar;
+  __shared__ __align__(8) unsigned long long s_bar[SEG];
 
   // Row of token t: below n0 the ring's (a block never wraps in it: its capacity is a multiple
   // of the block), else the caller's.
@@ -161,15 +164,20 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   auto row_of = [&](int t) -> const T* {
     return t < n_old ? ring_row0 + (size_t)t * TQ_D : in_row0 + (int64_t)t * src.tok_stride;
   };
-  // the block into shared memory: a bulk copy per row where rows are on the 16-byte grid, else
-  // element by element
+  // the block into shared memory: a bulk copy per row where rows are on the 16-byte grid (a barrier per
+  // segment, so that the first pass starts before the last rows are there), else element by element
   constexpr int ROW_BYTES = TQ_D * (int)sizeof(T);
   if (aligned) {
-    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
     if (tid == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+#pragma unroll
+      for (int s = 0; s < SEG; ++s)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * s) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(C::ROWS) : "memory");
+#pragma unroll
+      for (int s = 0; s < SEG; ++s)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 8 * s), "r"(C::ROWS / SEG)
+                     : "memory");
     }
     __syncthreads();
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ek_smem);
@@ -178,7 +186,7 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
               dst + tid * ROW_BYTES),
-          "l"(row_of(tid)), "r"(ROW_BYTES), "r"(bar)
+          "l"(row_of(tid)), "r"(ROW_BYTES), "r"(bar + 8 * (tid / NT))
           : "memory");
   } else {
     for (int i = tid; i < EK_S * TQ_D; i += THREADS) ((T*)ek_smem)[i] = row_of(i >> 7)[i & 127];
@@ -196,8 +204,8 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   if (tid < 16) s_grid[tid] = a.tables->grid[tid];
   if (tid == 0) s_n_redo = 0;
   for (int i = tid; i < EK_S * 4; i += THREADS) mask[i] = 0u;
-  auto landed = [&]() -> bool {  // bounded
-    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+  auto landed = [&](int s) -> bool {  // bounded
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar[s]);
     const int limit = a.wait_limit > 0 ? a.wait_limit : EK_WAIT;
     unsigned done = 0;
     for (int i = 0; i < limit && !done; ++i)
@@ -209,23 +217,26 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
           : "memory");
     return done != 0;
   };
-  if (__syncthreads_or(aligned && !landed())) {
-    // A copy did not arrive: nothing is encoded from rows that are not there.  The status word says
-    // so, the page becomes an empty one (scales, zero-points and corrections of zero), and the
-    // copies still on their way get another bounded wait before the CTA gives up its shared memory.
-    if (tid == 0) {
-      atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
-      a.page_meta[unit_index(g, a.layer, seq, head) * g.max_blocks + blk] = {0u, 0u};
-      landed();
+  // (last warp) for each bin the number of borders below its left edge; borders and bins in units
+  // where a channel spans [0, 1]
+  if (warp == THREADS / 32 - 1) {
+    const float level = a.tables->grid[lane & 15];
+    const float edge = ((float)lane - 0.5f) * (1.0f / (EK_BINS - 1)) - 5.0e-4f;
+    int cell = 0;
+    for (int l = 0; l < 15; ++l) {
+      const float here = __shfl_sync(0xffffffffu, level, l), next = __shfl_sync(0xffffffffu, level, l + 1);
+      const float b = mode == TQ_KEYS_UNIFORM ? ((float)l + 0.5f) * (1.0f / 15.0f) : 0.25f * (here + next) + 0.5f;
+      cell += b < edge ? 1 : 0;
     }
-    auto zero = [&](int from, int to) {  // (multiples of 16, as all parts of a page are)
-      for (int i = from + 16 * tid; i < to; i += 16 * THREADS) *(uint4*)(page + i) = make_uint4(0, 0, 0, 0);
-    };
-    zero(0, g.k_bytes);
-    zero(g.scale_off, g.page_bytes);
-    __syncthreads();
-    return;
+    // (above the last border: a huge one)
+    const float here = __shfl_sync(0xffffffffu, level, cell), next = __shfl_sync(0xffffffffu, level, min(cell + 1, 15));
+    s_bin[lane] = make_float4(here, next, __uint_as_float((uint32_t)cell), 0.0f);
   }
+  bool lost = false;
+  if (aligned)
+    lost = !landed(seg);
+  else
+    __syncthreads();
 
   // ---- pass 1: sum in token order, extremes, group maxima -------------------------------------
   // The sum is a chain over all tokens: a segment's threads take it over from the segment before
@@ -259,7 +270,7 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   };
   if (seg == 0 && mode == TQ_KEYS_NF4_ASYM) sum_segment();
   {
-    W* gmax = (W*)tab;  // [32 groups][64 pairs]
+    W* gmax = (W*)img;  // [32 groups][64 pairs]
     if constexpr (F32) {
       float2 mn = make_float2(INFINITY, INFINITY), mx = make_float2(-INFINITY, -INFINITY), gm[GPT];
 #pragma unroll
@@ -298,30 +309,64 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     }
   }
   if (seg > 0 && mode == TQ_KEYS_NF4_ASYM) sum_segment();
-  __syncthreads();
+  if (__syncthreads_or(lost)) {
+    // A copy did not arrive: nothing is encoded from rows that are not there.  The status word says
+    // so, the page becomes an empty one (scales, zero-points and corrections of zero), and the
+    // copies still on their way get another bounded wait before the CTA gives up its shared memory.
+    if (tid == 0) {
+      atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+      a.page_meta[unit_index(g, a.layer, seq, head) * g.max_blocks + blk] = {0u, 0u};
+      for (int s = 0; s < SEG; ++s) landed(s);
+    }
+    auto zero = [&](int from, int to) {  // (multiples of 16, as all parts of a page are)
+      for (int i = from + 16 * tid; i < to; i += 16 * THREADS) *(uint4*)(page + i) = make_uint4(0, 0, 0, 0);
+    };
+    zero(0, g.k_bytes);
+    zero(g.scale_off, g.page_bytes);
+    __syncthreads();
+    return;
+  }
 
-  // ---- per channel: zero-point, scale, bin mapping; the groups with the k largest maxima ---------
-  if (tid < TQ_D) {
-    const int d = tid;
+  // ---- per channel: zero-point, scale, bin mapping, table; the groups with the k largest maxima ------
+  // (a thread computes the zero-points and scales of the channels whose bins it fills: no barrier between)
+  auto channel = [&](int d, float& mu, float& amax) {
     float xmin = s_mn[d], xmax = s_mx[d];
 #pragma unroll
     for (int s = 1; s < SEG; ++s) {
       xmin = fminf(xmin, s_mn[s * TQ_D + d]);
       xmax = fmaxf(xmax, s_mx[s * TQ_D + d]);
     }
-    const float mu = mode == TQ_KEYS_NF4_ASYM
-                         ? (a.bias_means != nullptr
-                                ? a.bias_means[((size_t)blk * g.n_kv_heads + head) * TQ_D + d]
-                            : a.tables->mean_mask[d] ? __fdiv_rn(s_sum[d], (float)EK_S)
-                                                     : 0.0f)
-                     : mode == TQ_KEYS_NF4 ? 0.0f
-                                           : xmin;
+    mu = mode == TQ_KEYS_NF4_ASYM
+             ? (a.bias_means != nullptr ? a.bias_means[((size_t)blk * g.n_kv_heads + head) * TQ_D + d]
+                : a.tables->mean_mask[d] ? __fdiv_rn(s_sum[d], (float)EK_S)
+                                         : 0.0f)
+         : mode == TQ_KEYS_NF4 ? 0.0f
+                               : xmin;
     // (rounding is monotone: the largest |fl(x - mu)| is reached at an extreme)
-    float amax = mode == TQ_KEYS_NF4_ASYM
-                     ? fmaxf(fabsf(__fsub_rn(xmax, mu)), fabsf(__fsub_rn(xmin, mu)))
-                     : fmaxf(fabsf(xmax), fabsf(xmin));
+    amax = mode == TQ_KEYS_NF4_ASYM ? fmaxf(fabsf(__fsub_rn(xmax, mu)), fabsf(__fsub_rn(xmin, mu)))
+                                    : fmaxf(fabsf(xmax), fabsf(xmin));
     amax = fmaxf(amax, 1e-8f);
     if (mode == TQ_KEYS_UNIFORM) amax = __fdiv_rn(fmaxf(__fsub_rn(xmax, xmin), 1e-8f), 15.0f);
+  };
+  auto fill = [&](int d, float mu, float sc, int from, int to) {
+    uint32_t* col = tab + ek_col(d);
+#pragma unroll 4
+    for (int bin = from; bin < to; ++bin) {
+      const float4 b4 = s_bin[bin];
+      const uint32_t cell = __float_as_uint(b4.z);
+      const float l2 = 0.5f * (__fmul_rn(sc, b4.x) + __fmul_rn(sc, b4.y));
+      const float b = mode == TQ_KEYS_NF4 ? l2 : mu + l2;
+      // (the nearest number whose low bits are the code)
+      const int near16 = max((int)(__float_as_uint(b) & 0x7FFFFFFFu) + 8 - (int)cell, 0) & ~15;
+      col[bin * TQ_D] = cell < 15u ? (__float_as_uint(b) & 0x80000000u) | (uint32_t)near16 | cell
+                                   : 0x7F700000u | 15u;
+    }
+  };
+  constexpr int FILL0 = F32 ? 10 : 22;  // bins of the threads that also store the channel's numbers
+  if (tid < TQ_D) {
+    const int d = tid;
+    float mu, amax;
+    channel(d, mu, amax);
     s_mu[d] = mu;
     s_scale[d] = amax;
     ((float*)(page + g.scale_off))[d] = amax;
@@ -339,8 +384,9 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     const float range = mode == TQ_KEYS_UNIFORM ? 15.0f * amax : amax;
     const bool plain = range >= fabsf(mu) * (1.0f / 512.0f) && fabsf(mu) + range < 0x1p126f;
     s_tol[d] = plain ? (fabsf(mu) + range) * 0x1p-19f : INFINITY;
+    fill(d, mu, amax, 0, FILL0);
   } else if (!F32 && tid < TQ_D + 64) {  // packed: a thread per channel pair
-    const uint32_t* gm = (const uint32_t*)tab + (tid - TQ_D);
+    const uint32_t* gm = (const uint32_t*)img + (tid - TQ_D);
     uint32_t top[EK_K];
 #pragma unroll
     for (int j = 0; j < EK_K; ++j) top[j] = 0u;
@@ -365,7 +411,7 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     s_groups[2 * (tid - TQ_D) + 1] = hi;
   } else if (F32 && tid < 2 * TQ_D) {
     const int d = tid - TQ_D;
-    const float* gm = (const float*)tab + d;  // [32][128]
+    const float* gm = (const float*)img + d;  // [32][128]
     float top[EK_K];
 #pragma unroll
     for (int j = 0; j < EK_K; ++j) top[j] = 0.0f;
@@ -383,57 +429,17 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
 #pragma unroll
     for (int i = 0; i < EK_GROUPS; ++i) sel |= gm[i * TQ_D] >= low ? 1u << i : 0u;
     s_groups[d] = sel;
-  } else if (tid >= THREADS - 32) {
-    // (last warp) for each bin the number of borders below its left edge; borders and bins in
-    // units where a channel spans [0, 1]
-    const float edge = ((float)lane - 0.5f) * (1.0f / (EK_BINS - 1)) - 5.0e-4f;
-    int cell = 0;
-    for (int l = 0; l < 15; ++l) {
-      const float b = mode == TQ_KEYS_UNIFORM ? ((float)l + 0.5f) * (1.0f / 15.0f)
-                                              : 0.25f * (s_grid[l] + s_grid[l + 1]) + 0.5f;
-      cell += b < edge ? 1 : 0;
-    }
-    // (above the last border: a huge one)
-    s_bin[lane] = make_float4(s_grid[cell], s_grid[min(cell + 1, 15)], __uint_as_float((uint32_t)cell), 0.0f);
-  }
-  __syncthreads();
-
-  // ---- the table; meanwhile one warp ranks the four widest channels ---------------------------
-  {
-    const int d = tid & (TQ_D - 1);
-    const float sc = s_scale[d], mu = s_mu[d];
-    uint32_t* col = tab + ek_col(d);
-#pragma unroll 4
-    for (int bin = tid >> 7; bin < EK_BINS; bin += THREADS >> 7) {
-      const float4 b4 = s_bin[bin];
-      const uint32_t cell = __float_as_uint(b4.z);
-      const float l2 = 0.5f * (__fmul_rn(sc, b4.x) + __fmul_rn(sc, b4.y));
-      const float b = mode == TQ_KEYS_NF4 ? l2 : mu + l2;
-      // (the nearest number whose low bits are the code)
-      const int near16 = max((int)(__float_as_uint(b) & 0x7FFFFFFFu) + 8 - (int)cell, 0) & ~15;
-      col[bin * TQ_D] = cell < 15u ? (__float_as_uint(b) & 0x80000000u) | (uint32_t)near16 | cell
-                                   : 0x7F700000u | 15u;
-    }
-  }
-  if (warp == THREADS / 32 - 1) {  // largest scale first, ties to the lower channel
-    uint32_t key[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) key[i] = __float_as_uint(s_scale[4 * lane + i]);
-    for (int r = 0; r < TQ_WIDE; ++r) {
-      const uint32_t best = max(max(key[0], key[1]), max(key[2], key[3]));
-      const uint32_t top = __reduce_max_sync(0xffffffffu, best);
-      const int at = __ffs((int)__ballot_sync(0xffffffffu, best == top)) - 1;
-      if (lane == at) {
-        bool taken = false;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (!taken && key[i] == top) {
-            taken = true;
-            key[i] = 0u;
-            s_wide[r] = 4 * lane + i;
-          }
-      }
-      __syncwarp();
+  } else if (F32) {  // two threads a channel
+    const int d = tid & (TQ_D - 1), half = (tid >> 7) & 1;
+    float mu, amax;
+    channel(d, mu, amax);
+    fill(d, mu, amax, FILL0 + 11 * half, FILL0 + 11 * (half + 1));
+  } else {  // a thread per two channels
+#pragma unroll 1
+    for (int d = tid - 192; d < TQ_D; d += 64) {
+      float mu, amax;
+      channel(d, mu, amax);
+      fill(d, mu, amax, FILL0, EK_BINS);
     }
   }
   __syncthreads();
@@ -496,6 +502,28 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
   __syncthreads();
 
   // ---- elements close to a border; outliers -----------------------------------------------------
+  // (meanwhile the last warp ranks the four widest channels)
+  if (warp == THREADS / 32 - 1) {  // largest scale first, ties to the lower channel
+    uint32_t key[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) key[i] = __float_as_uint(s_scale[4 * lane + i]);
+    for (int r = 0; r < TQ_WIDE; ++r) {
+      const uint32_t best = max(max(key[0], key[1]), max(key[2], key[3]));
+      const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+      const int at = __ffs((int)__ballot_sync(0xffffffffu, best == top)) - 1;
+      if (lane == at) {
+        bool taken = false;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (!taken && key[i] == top) {
+            taken = true;
+            key[i] = 0u;
+            s_wide[r] = 4 * lane + i;
+          }
+      }
+      __syncwarp();
+    }
+  }
   {
     // The reference's nearest level: the first minimum of the rounded distances.  An element
     // close to a border has one of the two levels beside it (the code found, or a neighbour);
@@ -609,7 +637,18 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
 
-  PageHeader* hdr = (PageHeader*)(page + g.hdr_off);
+  // The page's tail is put together in shared memory and stored as one piece: slots, counts and codes of
+  // single tokens would be some forty scattered stores a warp.
+  uint8_t* tail = (uint8_t*)s_mn;
+  PageHeader* hdr = (PageHeader*)tail;
+  if (tid < TQ_SIDE_OFF / 4) ((uint32_t*)tail)[tid] = 0u;
+  else if (tid >= 64 && tid < 64 + TQ_OVF_CAP) ((uint32_t*)(tail + TQ_OVF_OFF))[tid - 64] = 0u;
+  auto store_tail = [&]() {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(page + g.hdr_off),
+                 "r"((uint32_t)__cvta_generic_to_shared(tail)), "r"(TQ_TAIL_BYTES)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  };
   // Exclusive prefix sums over the tokens of their outlier counts and of the counts beyond the
   // fixed slots (both in one word: each total stays below 65536); thread t owns token t.
   uint32_t mine = 0u, incl = 0u, m4[4] = {0u, 0u, 0u, 0u};
@@ -635,16 +674,19 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     for (int w = 0; w < EK_S / 32; ++w) sum += s_scan[w];
     n_out = (int)(sum & 0xffffu);
   }
-  if (tid == THREADS - 32) {
-    // this page's slice of the (layer, seq, head) outlier slab
+  // This page's slice of the (layer, seq, head) outlier slab.  (Its place is not waited for until the
+  // page's own lists are written.)
+  uint32_t pool_at = 0u;
+  if (tid == THREADS - 32 && n_out > 0)
+    pool_at = atomicAdd(&a.pool_cursor[unit_index(g, a.layer, seq, head)], (uint32_t)((n_out + 3) & ~3));
+  auto take_slice = [&]() {
     uint32_t sum = 0u;
     for (int w = 0; w < EK_S / 32; ++w) sum += s_scan[w];
     const int n = n_out, n_ovf = (int)(sum >> 16);
-    uint32_t off = 0;
+    uint32_t off = pool_at;
     int alloc = 0;
     if (n > 0) {
       const int n4 = (n + 3) & ~3;
-      off = atomicAdd(&a.pool_cursor[unit_index(g, a.layer, seq, head)], (uint32_t)n4);
       if (off >= (uint32_t)g.pool_entries) off = 0;
       else alloc = min(n4, g.pool_entries - (int)off);
       if (alloc < n4) atomicOr(a.status, TQ_STATUS_POOL_OVERFLOW);
@@ -662,10 +704,10 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
     hdr->flags = (n_ovf > TQ_OVF_CAP || alloc < n) ? TQ_PAGE_SPILLED : 0;
     s_off_pool = off;
     s_alloc = alloc;
-  }
-  uint16_t* ell_delta = (uint16_t*)(page + g.hdr_off + TQ_ELL_OFF);  // [slot][token]
-  uint8_t* ell_col = page + g.hdr_off + TQ_ELL_COL_OFF;               // [slot][token]
-  uint32_t* ovf = (uint32_t*)(page + g.hdr_off + TQ_OVF_OFF);
+  };
+  uint16_t* ell_delta = (uint16_t*)(tail + TQ_ELL_OFF);  // [slot][token]
+  uint8_t* ell_col = tail + TQ_ELL_COL_OFF;               // [slot][token]
+  uint32_t* ovf = (uint32_t*)(tail + TQ_OVF_OFF);
   int row = 0;  // where this token's outliers start
   if (tid < EK_S) {
     uint32_t excl = incl - mine;
@@ -687,15 +729,16 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
       const int d = s_wide[r];
       side |= (uint32_t)((img[tid * (TQ_D / 2) + (d >> 1)] >> (4 * (d & 1))) & 15) << (4 * r);
     }
-    ((uint16_t*)(page + g.hdr_off + TQ_SIDE_OFF))[tid] = (uint16_t)side;
+    ((uint16_t*)(tail + TQ_SIDE_OFF))[tid] = (uint16_t)side;
   }
   if (tid < TQ_WIDE) hdr->wide[tid] = (uint8_t)s_wide[tid];
   // The outliers by token, then channel (the order of the reference's flat indices), listed in
   // shared memory and stored one per thread; in several rounds where there are more than fit.
   unsigned short* list = (unsigned short*)tab;  // token | channel << 8
   constexpr int LIST = C::TAB / 2;
+  constexpr int PRE = 4;  // entries of a thread that are ready before the slice is known
   for (int base = 0; base < n_out; base += LIST) {
-    __syncthreads();
+    if (base > 0) __syncthreads();
     if (cnt > 0) {
       int i = row - base;
 #pragma unroll
@@ -704,10 +747,8 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
           if (i >= 0 && i < LIST) list[i] = (unsigned short)(tid | ((32 * w + __ffs((int)left) - 1) << 8));
     }
     __syncthreads();
-    const int alloc = s_alloc, n = min(n_out - base, LIST);
-    const size_t slab = unit_index(g, a.layer, seq, head) * (size_t)g.pool_entries + s_off_pool;
-#pragma unroll 2
-    for (int i = tid; i < n; i += THREADS) {
+    const int n = min(n_out - base, LIST);
+    auto entry = [&](int i) -> uint2 {  // (the pool's two words); and to the page
       const int t = list[i] & 255, d = list[i] >> 8, slot = base + i, below = slot - (int)s_row[t];
       const float v = Elem<DT>::ld(rows, t * TQ_D + d);
       const int code = (img[t * (TQ_D / 2) + (d >> 1)] >> (4 * (d & 1))) & 15;
@@ -716,10 +757,6 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
       const float dense = mode == TQ_KEYS_NF4 ? sl : __fadd_rn(s_mu[d], sl);
       const __half delta = __float2half_rn(__fsub_rn(__half2float(hv), dense));
       const uint32_t ent = (uint32_t)__half_as_ushort(delta) | ((uint32_t)d << 16) | ((uint32_t)t << 24);
-      if (slot < alloc) {
-        a.pool_dec[slab + slot] = ent;
-        a.pool_val[slab + slot] = __half_as_ushort(hv);
-      }
       if (below < TQ_ELL_SLOTS) {
         ell_delta[below * 256 + t] = __half_as_ushort(delta);
         ell_col[below * 256 + t] = (uint8_t)q_row(d);
@@ -727,7 +764,36 @@ __global__ void __launch_bounds__(Ek<DT>::THREADS, DT == TQ_F32 ? 1 : 2)
         const int oi = (int)s_orow[t] + below - TQ_ELL_SLOTS;
         if (oi < TQ_OVF_CAP) ovf[oi] = ent;
       }
+      return make_uint2(ent, __half_as_ushort(hv));
+    };
+    uint2 pre[PRE];
+#pragma unroll
+    for (int j = 0; j < PRE; ++j)
+      if (tid + j * THREADS < n) pre[j] = entry(tid + j * THREADS);
+    if (base == 0) {
+      if (tid == THREADS - 32) take_slice();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+      if (n_out <= PRE * THREADS && tid == THREADS - 1) store_tail();
     }
+    const int alloc = s_alloc;
+    const size_t slab = unit_index(g, a.layer, seq, head) * (size_t)g.pool_entries + s_off_pool + base;
+    auto store = [&](int i, uint2 e) {
+      if (base + i < alloc) {
+        a.pool_dec[slab + i] = e.x;
+        a.pool_val[slab + i] = (uint16_t)e.y;
+      }
+    };
+#pragma unroll
+    for (int j = 0; j < PRE; ++j)
+      if (tid + j * THREADS < n) store(tid + j * THREADS, pre[j]);
+    for (int i = tid + PRE * THREADS; i < n; i += THREADS) store(i, entry(i));
+  }
+  if (n_out == 0 || n_out > PRE * THREADS) {
+    if (n_out == 0 && tid == THREADS - 32) take_slice();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (tid == THREADS - 1) store_tail();
   }
   if (tid == THREADS - 1)  // the image has been read before the CTA gives its shared memory back
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
