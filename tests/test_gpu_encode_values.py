@@ -125,3 +125,23 @@ def test_polar_keys_take_the_same_tiles():
     v = torch.randn((1, 1300, 2, 128), generator=gen, device="cuda").half()
     a, b = _values(v, (700, 600), 2, 4, 512, "float16", key_mode="polar")
     assert a == b
+
+
+@pytest.mark.parametrize("vb,outer", [(3, 0.3), (4, 0.25)])
+def test_codebook_wider_than_the_table(vb, outer, monkeypatch):
+    """A caller's codebook whose boundaries crowd in the middle leaves no range in which 32 bins part all of
+    them: the table must not be used with the outer ones beyond its range."""
+    import torch
+
+    from turboquant_pro_b200 import context
+
+    n = 2**vb
+    inner = 0.004 * (np.arange(n - 3) - (n - 4) / 2)
+    bounds = np.concatenate([[-outer], inner, [outer]]).astype(np.float32)
+    cents = np.concatenate([[-0.4], (bounds[1:] + bounds[:-1]) / 2, [0.4]]).astype(np.float32)
+    monkeypatch.setattr(context, "value_codebook", lambda head_dim, bits: (cents, bounds))
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(6)
+    v = torch.randn((1, 1500, 2, 128), generator=gen, device="cuda").half()
+    a, b = _values(v, (1500,), 2, vb, 512, "float16")
+    assert a == b

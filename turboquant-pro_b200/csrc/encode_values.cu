@@ -780,7 +780,8 @@ int launch_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys, int
 }  // namespace
 
 void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable* vt) {
-  // the widest range of y whose 32 bins hold at most one boundary each, with the slack on both sides
+  // the widest range of y that holds all boundaries and whose 32 bins hold at most one each, with the slack
+  // on both sides
   const int n = (1 << bits) - 1;
   vt->ok = false;
   for (int i = 0; i < n; ++i)
@@ -789,23 +790,28 @@ void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable*
     const double unit = VALUE_SPAN * 8388608.0 / (2.0 * range);  // Z per y
     const long slack = (long)std::ceil(value_slack(kv_dtype) * unit) + 2;
     long at[15];
-    for (int i = 0; i < n; ++i) at[i] = std::lround((boundaries[i] + range) * unit);
+    int touched = 0;  // last bin the boundaries so far can lie in; the first and the last bin have none
     bool fits = slack < (1 << 17);
-    for (int k = 0; k < 32 && fits; ++k) {
+    for (int i = 0; i < n && fits; ++i) {
+      at[i] = std::lround((boundaries[i] + range) * unit);
+      const long first = ((at[i] - 2 * slack + (1 << 18) - 1) >> 18) - 1;
+      fits = first > touched;
+      touched = (int)((at[i] + 2 * slack) >> 18);
+    }
+    if (!fits || touched > 30) continue;
+    const int sh = 32 - bits;
+    for (int k = 0; k < 32; ++k) {
       const long lo = (long)k << 18, hi = lo + (1 << 18);
-      int below = 0, inside = 0, which = 0;
+      int below = 0, which = -1;
       for (int i = 0; i < n; ++i) {
-        if (at[i] >= lo - 2 * slack && at[i] <= hi + 2 * slack) ++inside, which = i;
+        if (at[i] >= lo - 2 * slack && at[i] <= hi + 2 * slack) which = i;
         else if (at[i] < lo) ++below;
       }
-      // (the first and the last bin also take what lies out of range)
-      fits = inside <= (k == 0 || k == 31 ? 0 : 1);
-      const int sh = 32 - bits;
-      const int64_t base = inside ? ((int64_t)(which + 1) << sh) - at[which]
-                                  : ((int64_t)below << sh) + (1ll << (sh - 1)) - lo;
+      const int64_t base = which >= 0 ? ((int64_t)(which + 1) << sh) - at[which]
+                                      : ((int64_t)below << sh) + (1ll << (sh - 1)) - lo;
       vt->off[k] = (int32_t)(uint32_t)(base - 0x3F800000ll);
     }
-    vt->ok = fits;
+    vt->ok = true;
     vt->slack = (uint32_t)slack;
     vt->scale = (float)(1.0 / (2.0 * range));
     vt->zero_code = 0u;
