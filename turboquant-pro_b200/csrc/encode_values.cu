@@ -480,7 +480,9 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     const uint32_t near_add = vt.slack << VB, near_lim = 2u * near_add;
     const int ew = warp - EV_LOADERS / 32;
     EvList& li = sh.list[ew];
-    int put = 0, told = 0;  // entries written, and told to the warp that takes them
+    // entries written, told to the warp that takes them, and taken by it as far as this warp knows (the
+    // same in every lane)
+    int put = 0, told = 0, seen = 0;
     auto publish = [&]() {
       __syncwarp();
       if (lane == 0) {  // (a group's codes are in the page before its entries are seen)
@@ -571,15 +573,20 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
         unsigned todo = __ballot_sync(0xffffffffu, near != 0u);
         while (todo) {
           const int n = __popc(todo);
-          if (put + n - *(volatile int*)&sh.got[ew] > EV_LIST && put != told) publish();
-          for (int k = 0; !gave_up && put + n - *(volatile int*)&sh.got[ew] > EV_LIST; ++k) {
-            if (k >= EV_WAIT) {
-              atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
-              gave_up = true;
+          if (put + n - seen > EV_LIST) {
+            if (put != told) publish();
+            for (int k = 0;; ++k) {
+              // (one lane's reading, so that the warp decides as one: the taking warp writes it meanwhile)
+              seen = __shfl_sync(0xffffffffu, *(volatile int*)&sh.got[ew], 0);
+              if (gave_up || put + n - seen <= EV_LIST) break;
+              if (k >= EV_WAIT) {
+                if (lane == 0) atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+                gave_up = true;
+              }
+              __nanosleep(100);
             }
-            __nanosleep(100);
+            __threadfence_block();  // (what those entries held has been read)
           }
-          gave_up = __any_sync(0xffffffffu, gave_up);
           if (gave_up) break;
           if (near) {
             const int b = __ffs((int)near) - 1, j = b & 7, jj = j & 3;
