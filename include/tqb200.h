@@ -410,12 +410,15 @@ int32_t tq_set_kernel(tq_ctx* ctx, int32_t which);
  * kv_fused_pck.py:216-236); no direct counterpart. */
 int32_t tq_last_kernel(const tq_ctx* ctx);
 
-/* Test hook for the bounded waits of the tensor-core decode kernel and of the key encoder for
- * 256-token blocks (no counterpart in the reference).  `wait_limit` > 0 replaces the number of
- * probes a wait makes before it gives up (0 restores the defaults, at most about half a second);
+/* Test hook for the bounded waits of the tensor-core decode kernel, of the key encoder for
+ * 256-token blocks and of the value encoder for 128- and 256-token blocks (no counterpart in the
+ * reference).  `wait_limit` > 0 replaces the number of
+ * probes a wait makes before it gives up (0 restores the defaults, a few seconds at most);
  * `withhold_tile` >= 0 makes the first CTA of later decodes never start the copy of that tile of
  * its share, and the first CTA of later appends that of the row of that number of its block, so
  * that the wait for it runs out and bit 1 of the status word is set (-1 switches this off).
+ * 2^20 + i stands for the products of the i-th tile of the value encoder's first CTA.  A block or tile
+ * that was not encoded is stored as zeros.
  * Nothing faults and nothing spins without bound; used by the tests of the error path. */
 int32_t tq_debug_wait(tq_ctx* ctx, int32_t wait_limit, int32_t withhold_tile);
 

@@ -23,3 +23,44 @@ def test_every_product_listed(dt, scale, vb):
         v *= scale
     a, b = _values(v.to(getattr(torch, dt)), (700, 700), 3, vb, 512, dt)
     assert a == b
+
+
+@pytest.mark.parametrize("dt,vb", [("float16", 3), ("bfloat16", 4), ("float32", 4)])
+def test_a_tile_that_is_not_encoded_is_stored_as_zeros(dt, vb):
+    """The test hook withholds the products of the first CTA's second tile; the waits for them run out, the
+    status word says so, and that tile and the CTA's later ones are rows of zeros, the others as ever."""
+    import torch
+
+    from turboquant_pro_b200 import KVContext
+
+    h, blocks, n = 8, 20, 512 + 20 * 256
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(10)
+    x = torch.randn((1, n, h, 128), generator=gen, device="cuda").to(getattr(torch, dt))
+    good, ctx = (KVContext(n_layers=1, n_seqs=1, n_kv_heads=h, n_q_heads=h, value_bits=vb,
+                           hot_window=512, max_tokens_per_seq=n, kv_dtype=dt, seed=5)
+                 for _ in range(2))
+    good.append(0, x, x)
+    want_k, want = good.dequant(0, 0, 0, n)
+    ctx._regions["pages"].fill_(0x5A)  # what an earlier user of the pages left there
+    ctx.debug_wait(wait_limit=512, withhold_tile=(1 << 20) + 1)
+    ctx.append(0, x, x)
+    assert ctx.status() == 2 and ctx.status() == 0
+    ctx.debug_wait()
+    k, v = ctx.dequant(0, 0, 0, n)
+    assert torch.equal(k, want_k)
+    tile = 64 if dt == "float32" else 128
+    parts, ctas = 256 // tile, torch.cuda.get_device_properties(0).multi_processor_count
+    lost = torch.zeros((h, n), dtype=torch.bool, device="cuda")
+    for w in range(ctas, h * blocks * parts, ctas):
+        head, t = w // (blocks * parts), w % (blocks * parts) * tile
+        lost[head, t:t + tile] = True
+    assert lost.any() and not v[lost].any() and torch.equal(v[~lost], want[~lost])
+    for head, t in lost.nonzero()[::tile].tolist():
+        codes = ctx.export_block(0, 0, t // 256)["value_indices"]
+        row = 128 * vb // 8
+        at = (head * 256 + t % 256) * row
+        assert not codes.reshape(-1)[at:at + row].any()
+    ctx.clear(0, 0)
+    ctx.append(0, x, x)
+    assert ctx.status() == 0 and torch.equal(ctx.dequant(0, 0, 0, n)[1], want)

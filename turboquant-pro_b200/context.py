@@ -735,9 +735,8 @@ class KVContext:
         return {0: "none", 1: "tensor-core", 2: "general"}[int(self._lib.tq_last_kernel(self._h))]
 
     def debug_wait(self, wait_limit: int = 0, withhold_tile: int = -1) -> None:
-        """Test hook of the bounded waits of the decode kernel and the key encoder: a shorter probe
-        limit and a tile (a row) of the first CTA whose copy is never started (see
-        ``tq_debug_wait``)."""
+        """Test hook of the bounded waits of the decode kernel and the encoders: a shorter probe limit
+        and a tile (a row) of the first CTA that is never started (see ``tq_debug_wait``)."""
         check(self._lib.tq_debug_wait(self._h, int(wait_limit), int(withhold_tile)))
 
     def trace(self, on: bool, read: bool = False):

@@ -35,7 +35,7 @@ constexpr int TQ_PAGE_SPILLED = 1;  // header flag: use the pool's list, not the
 
 // device status word: bit 0, an outlier pool overflowed; bit 1, a bounded wait ran out: of the
 // tensor-core decode kernel (the call's output is then undefined) or of an encoder (the append then
-// stored a block that does not hold its tokens)
+// stored zeros in place of a block or of a tile of one)
 constexpr int TQ_STATUS_POOL_OVERFLOW = 1;
 constexpr int TQ_STATUS_WAIT_TIMEOUT = 2;
 constexpr int TQ_STATUS_BAD_PAGE = 4;  // a page id outside the engine's tensor; its tokens were left out
@@ -125,7 +125,7 @@ struct tq_ctx {
   int last_q_dtype = TQ_F32;   // query element type of the most recent decode (byte accounting)
   bool force_generic = false;  // route every decode through the general-shape kernel
   bool trace_on = false;       // the tensor-core decode kernel stamps its pipeline phases
-  int wait_limit = 0;          // probes per bounded wait of the decode kernel and the key encoder; 0 = default
+  int wait_limit = 0;          // probes per bounded wait of the decode kernel and the encoders; 0 = default
   int withhold_tile = -1;      // test hook: the copy of this tile (key encoder: row) of CTA 0 is never started
   // optional per-kernel timing: event triples (before attention, after it, after combine)
   bool prof_on = false;

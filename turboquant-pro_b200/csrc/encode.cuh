@@ -24,8 +24,9 @@ struct EncodeArgs {
   // PolarQuant keys (TQ_KEYS_POLAR): the value encoder also runs over the keys, writing their
   // codes where the per-channel codes would go and their norms over the scale / mean arrays
   int polar_keys_pass;
-  // bounded waits of the key encoder: probes (0: its default); test hook: the row of the first new
-  // block whose copy is never started (-1: none)
+  // bounded waits of the encoders: probes (0: their defaults); test hook: the row of the first new
+  // block whose copy the key encoder never starts, or 2^20 + the tile whose products the first CTA of the
+  // value encoder never starts (-1: none)
   int wait_limit, withhold_row;
 };
 

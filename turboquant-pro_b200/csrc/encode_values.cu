@@ -36,6 +36,7 @@
 // (switched off: 165 us without lists and their recomputation, 124 without codes, products and norms, 83
 // without the copies, too); 42 % of the issue slots, six warps a scheduler.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "encode.cuh"
@@ -59,8 +60,8 @@ constexpr int EV_PER_REDO = EV_EPI_WARPS / EV_REDO_WARPS;  // lists a redo warp 
 constexpr int EV_LIST = 64;                  // entries of a list (a ring)
 constexpr int EV_PI_BYTES = 2 * TQ_D * TQ_D * 2;
 constexpr int EV_TILE_BYTES = 33280;         // rows of a tile: 128 x 256 or 64 x 512 bytes, and the pads
-constexpr int EV_WAIT = 1 << 20;             // probes of a barrier before a wait gives up
-constexpr int EV_POLLS = 1 << 25;            // idle polls before a redo warp gives up
+constexpr int EV_WAIT = 1 << 20;             // probes of a barrier (2 us each at most) before a wait gives up
+constexpr int EV_WITHHOLD = 1 << 20;         // test hook: a.withhold_row of tile 0 of the first CTA
 
 template <int DT>
 struct EvShape {
@@ -99,6 +100,7 @@ struct EvShared {
   unsigned long long odd[4];  // per slot, a byte per loader warp: it has a token without a usable norm
   unsigned long long full[4], done[4], empty[4];
   uint32_t tmem;
+  int lost;  // first tile whose codes or norms are not all there: a wait ran out
 };
 static_assert(sizeof(EvShared) <= 227 * 1024, "shared memory of one CTA");
 
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   }
   if (threadIdx.x < EV_EPI_WARPS)
     sh.put[threadIdx.x] = sh.got[threadIdx.x] = sh.fin[threadIdx.x] = 0;
+  if (threadIdx.x == 0) sh.lost = INT_MAX;
   if (warp == 0) {
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -225,6 +228,11 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *(volatile uint32_t*)&sh.tmem;
 
+  const int limit = a.wait_limit > 0 ? min(a.wait_limit, 1 << 26) : EV_WAIT;
+  auto lose = [&](int i) {  // a wait for tile i ran out
+    atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+    atomicMin(&sh.lost, i);
+  };
   bool gave_up = false;  // (no later wait of this thread probes again)
   // bounded wait for the phase of `bars` that tile i completes
   auto wait = [&](unsigned long long* bars, int i) {
@@ -232,8 +240,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     const uint32_t bar = enc_smem(&bars[i % SLOTS]);
     const unsigned parity = (unsigned)((i / SLOTS) & 1);
     for (int n = 0; !mbar_try_wait(bar, parity);) {
-      if (++n >= EV_WAIT) {
-        atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+      if (++n >= limit) {
+        lose(i);
         gave_up = true;
         break;
       }
@@ -336,6 +344,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(T >> 3) << 17) |
                                ((128u >> 4) << 24);
     auto issue = [&](int i) {
+      if (blockIdx.x == 0 && a.withhold_row - EV_WITHHOLD == i) return;  // test hook
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + (uint32_t)((i % SLOTS) * T);
       const uint64_t a_hi0 = umma_desc_k_major(enc_smem(sh.pi), 2048, 128);
@@ -466,8 +475,10 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     if (n >= SLOTS) wait(sh.empty, n - SLOTS);
     if (tl == 0) sh.info[n & 3].dst = nullptr;
     mbar_arrive(enc_smem(&sh.full[n % SLOTS]));
-    gave_up = false;
-    if (n > 0) wait(sh.done, n - 1);  // no product is under way when the tensor memory goes back
+    for (int i = max(n - SLOTS, 0); i < n; ++i) {  // no product is under way when the tensor memory goes back
+      gave_up = false;
+      wait(sh.done, i);
+    }
   } else if (warp < EV_LOADERS / 32 + EV_EPI_WARPS) {
     // ---- epilogue --------------------------------------------------------------------------
     // tensor-memory lanes 32 wq on; of the groups of all tiles every third
@@ -579,8 +590,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
               // (one lane's reading, so that the warp decides as one: the taking warp writes it meanwhile)
               seen = __shfl_sync(0xffffffffu, *(volatile int*)&sh.got[ew], 0);
               if (gave_up || put + n - seen <= EV_LIST) break;
-              if (k >= EV_WAIT) {
-                if (lane == 0) atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+              if (k >= 16 * limit) {
+                if (lane == 0) lose(i);
                 gave_up = true;
               }
               __nanosleep(100);
@@ -675,8 +686,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
       }
       __threadfence_block();
       if (total < 32 && !all_fin) {
-        if (++idle >= EV_POLLS) {
-          if (lane == 0) atomicOr(a.status, TQ_STATUS_WAIT_TIMEOUT);
+        if (++idle >= 4 * limit) {
+          if (lane == 0) lose(0);
           break;
         }
         __nanosleep(2000);
@@ -748,6 +759,24 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Sh::COLS)
                  : "memory");
+  }
+  if (sh.lost != INT_MAX) {
+    // What a wait gave up on, and this CTA's tiles after it, are stored as rows of zeros: the pages may hold
+    // anything where no codes were written.
+    int i = 0;
+    for (long w = blockIdx.x;; w += gridDim.x) {
+      const int parts = g.block_tokens / T, part = (int)(w % parts), jb = (int)(w / parts % a.max_new_blocks);
+      const long unit = w / parts / a.max_new_blocks;
+      if (unit >= (long)a.seq_count * g.n_kv_heads) break;
+      const int head = (int)(unit % g.n_kv_heads), seq = a.seq_begin + (int)(unit / g.n_kv_heads);
+      const int n0 = a.seq_len[a.layer * g.n_seqs + seq];
+      const int blk = n_cold_blocks(n0, g.hot_window, g.block_tokens) + jb;
+      if (blk >= n_cold_blocks(n0 + a.n_tokens, g.hot_window, g.block_tokens) || i++ < sh.lost) continue;
+      uint8_t* page = a.pages + page_offset(g, a.layer, seq, head, blk);
+      uint4* codes = (uint4*)(page + out_off + (size_t)part * (T / TQ_GROUP_TOK) * VGB);
+      for (int k = threadIdx.x; k < T / TQ_GROUP_TOK * VGB / 16; k += EV_THREADS) codes[k] = make_uint4(0, 0, 0, 0);
+      if (threadIdx.x < T) ((float*)(page + nrm_off))[part * T + threadIdx.x] = 0.0f;
+    }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");  // (the kernel before this one, see the launch)
 }
