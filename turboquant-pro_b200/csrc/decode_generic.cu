@@ -462,7 +462,8 @@ __global__ void __launch_bounds__(TQ_D) combine_kernel(DecodeArgs a) {
   float M = -INFINITY;
 #pragma unroll 8
   for (int s = 0; s < ns; ++s) M = fmaxf(M, s_m[s]);
-  if (e < ns) s_w[e] = s_m[e] > -INFINITY ? __expf(s_m[e] - M) : 0.0f;
+  const bool log2 = tq_decode_pages_form(g);  // (the unit of the maxima)
+  if (e < ns) s_w[e] = !(s_m[e] > -INFINITY) ? 0.0f : log2 ? tq_exp2(s_m[e] - M) : __expf(s_m[e] - M);
   __syncthreads();
   float L = 0.0f, C = 0.0f, Hh = 0.0f;
   auto add = [&](int s, float y) {
@@ -480,15 +481,21 @@ __global__ void __launch_bounds__(TQ_D) combine_kernel(DecodeArgs a) {
   for (int s = FIRST; s < ns; ++s) add(s, base[s * stride + 2 + e]);
   cs[e] = C;
   __syncthreads();
-  float o = 0.0f;
-#pragma unroll 32
-  for (int d = 0; d < TQ_D; ++d) o += cs[d] * a.tables->pi[d * TQ_D + e];
+  // (eight sums: a chain of 128 rounded additions would be the largest part of the error)
+  float o8[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o8[i] = 0.0f;
+#pragma unroll 4
+  for (int d = 0; d < TQ_D; d += 8)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o8[i] += cs[d + i] * a.tables->pi[(d + i) * TQ_D + e];
+  const float o = ((o8[0] + o8[1]) + (o8[2] + o8[3])) + ((o8[4] + o8[5]) + (o8[6] + o8[7]));
   const size_t row = (size_t)seq * g.n_q_heads + head * G + gg;
   const float val = o + Hh;
   if (a.mlo != nullptr) {
     float* r = a.mlo + row * TQ_PART_STRIDE;
     if (e == 0) {
-      r[0] = M;
+      r[0] = log2 ? tq_scaled<false>(M) : M;
       r[1] = L;
     }
     r[2 + e] = val;

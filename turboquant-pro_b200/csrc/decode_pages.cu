@@ -4,10 +4,17 @@
 // through its combine kernel.
 //
 // The products run on mma.sync tiles (m16n8k16, eight query heads across) with every float32 operand
-// split into two fp16 parts, x = hi + lo: 22 bits and the sign, scaled by powers of two so that lo keeps
-// its bits.  hi * hi + hi * lo + lo * hi leaves out 2^-24 of a term; the three products of a 16-deep
-// step start from zero and are added up in float32 registers with ordinary rounding (a chain
-// inside the tensor cores would truncate at every step).
+// split into two fp16 parts, x = hi + lo, good to 2^-23 of x.  Powers of two keep lo in fp16's range: a head's
+// weights are scaled by their largest, a head's probabilities times norms by the strip's largest such
+// product.  (By its largest norm alone, as this once was, lo and then hi drop out where a token with
+// a small value dominates the softmax: 1.7e-2 of the output with 24 nats between the two.)  An operand
+// that is itself a product is split before it is rounded.  hi * hi + hi * lo + lo * hi leaves out 2^-22 of a
+// term at most.  The tensor cores cut sums off where float32 rounds them, so of the scores only hi * hi
+// of 16 channels is summed there; these are added up in float32, and the small products have a sum of
+// their own.  Scores are in units of log 2 (decode_generic.cuh).
+// Distance from 64 bits, plain float32 multiply-adds / this, 24 caches of 700 and 3 000 tokens at seven heads:
+// 4.8e-7 / 4.5e-7 and 6.2e-7 / 5.6e-7; queries three times as large 6.2e-7 / 5.7e-7 and 7.6e-7 / 7.4e-7; a
+// token without a value 24 nats above the rest 1.65e-6 / 1.50e-6.
 //
 // Persistent CTAs of three groups of four warps, one CTA an SM.  The pages of all sequences, heads and
 // head tiles form one list that is cut into equal shares, one per group, so ragged batches balance;
@@ -121,6 +128,13 @@ TQ_DEV void dp_split(float a, float b, uint32_t& hi, uint32_t& lo) {
   hi = *(const uint32_t*)&h;
   lo = dp_h2(a - f.x, b - f.y);
 }
+// the same of a * x and b * y: lo takes what the products' rounding would drop, too
+TQ_DEV void dp_split_products(float a, float x, float b, float y, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(a * x, b * y);
+  const float2 f = __half22float2(h);
+  hi = *(const uint32_t*)&h;
+  lo = dp_h2(fmaf(a, x, -f.x), fmaf(b, y, -f.y));
+}
 TQ_DEV uint2 dp_lut(uint32_t addr) {  // (the tables never change: not volatile)
   uint2 v;
   asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
@@ -134,7 +148,8 @@ TQ_DEV void dp_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]),
         "f"(c[2]), "f"(c[3]));
 }
-// d = a * b of one 16-deep step, the small products first
+// d = a * b of one 16-deep step, the small products first: a sum that starts from zero and goes on in
+// float32 registers
 TQ_DEV void dp_product(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4],
                        const uint32_t (&bh)[2], const uint32_t (&bl)[2]) {
   const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -253,15 +268,15 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
   share = max(share, a.ns_cold > 2 ? (most + a.ns_cold - 4) / (a.ns_cold - 2) : most);
   share = max(share, 1);
 
-  // the query rows of a tile
-  auto load_q = [&](int unit, int gt) {
+  // the query rows of a tile; `log2`: times the scores' unit
+  auto load_q = [&](int unit, int gt, bool log2) {
     const int seq = unit / H, head = unit - seq * H;
 #pragma unroll
     for (int gg = 0; gg < GT; ++gg) {
       const int qh = gt * GT + gg;
-      q_s[q_row(gtid)][gg] = qh < G ? dp_ld(a.q, ((size_t)seq * g.n_q_heads + head * G + qh) * TQ_D + gtid,
-                                            a.q_dtype)
-                                    : 0.0f;
+      const size_t at = ((size_t)seq * g.n_q_heads + head * G + qh) * TQ_D + gtid;
+      const float x = qh < G ? dp_ld(a.q, at, a.q_dtype) : 0.0f;
+      q_s[q_row(gtid)][gg] = log2 ? tq_scaled<true>(x) : x;
     }
   };
   auto slot_of = [&](int unit, int gt, int slot) -> float* {
@@ -357,7 +372,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
       float M = -INFINITY;
 #pragma unroll
       for (int w = 0; w < 4; ++w) M = fmaxf(M, sh.m[gi][w][2 * c + x]);
-      f[x] = m_run[x] > -INFINITY ? __expf(m_run[x] - M) : 0.0f;
+      f[x] = m_run[x] > -INFINITY ? tq_exp2(m_run[x] - M) : 0.0f;
     }
     float* sums = &sh.corr[gi][0][0][0];  // [8 heads][128], bits 3 and 4 of the channel by the head
     for (int w = 0; w < 4; ++w) {
@@ -385,7 +400,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
       for (int w = 0; w < 4; ++w) M = fmaxf(M, sh.m[gi][w][gtid]);
 #pragma unroll
       for (int w = 0; w < 4; ++w)
-        L += sh.m[gi][w][gtid] > -INFINITY ? sh.l[gi][w][gtid] * __expf(sh.m[gi][w][gtid] - M) : 0.0f;
+        L += sh.m[gi][w][gtid] > -INFINITY ? sh.l[gi][w][gtid] * tq_exp2(sh.m[gi][w][gtid] - M) : 0.0f;
       pp[gtid * TQ_PART_STRIDE] = M;
       pp[gtid * TQ_PART_STRIDE + 1] = L;
     }
@@ -423,7 +438,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
       const int unit = (seq0 + p.seq) * H + p.row / tiles, gt = p.row % tiles;
       if (fresh) {
         group_sync();  // (the queries and sums of the row before are no longer read)
-        load_q(unit, gt);
+        load_q(unit, gt, true);
         reset();
         group_sync();
         fresh = false;
@@ -466,8 +481,10 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          dp_split(w[j][0] * up, w[j][1] * up, bh[j][0], bl[j][0]);
-          dp_split(w[j][2] * up, w[j][3] * up, bh[j][1], bl[j][1]);
+          const float4 s4 = *(const float4*)&st.scale[c][4 * j];  // (again: w is rounded)
+          const int d = 32 * c + 4 * j;
+          dp_split_products(q_s[q_row(d)][r] * up, s4.x, q_s[q_row(d + 1)][r] * up, s4.y, bh[j][0], bl[j][0]);
+          dp_split_products(q_s[q_row(d + 2)][r] * up, s4.z, q_s[q_row(d + 3)][r] * up, s4.w, bh[j][1], bl[j][1]);
         }
       }
 
@@ -532,7 +549,9 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
             const uint4 v = *(const uint4*)(st.keys + (16 * h + 8 * x + r) * (TQ_D / 2) + c * 16);
             kw[x][0] = v.x, kw[x][1] = v.y, kw[x][2] = v.z, kw[x][3] = v.w;
           }
-          float sum[2][4];
+          // hi * hi a step at a time, the products with a low part in one sum of their own
+          float sum[2][4], low[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             uint32_t ah[4], al[4];
@@ -543,16 +562,17 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
               ah[x] = t.x, al[x] = t.y;
             }
             float d[4];
-            dp_product(d, ah, al, bh[j], bl[j]);
+            dp_mma(d, ah, bh[j][0], bh[j][1], zero);
+            dp_mma(low, al, bh[j][0], bh[j][1], low);
+            dp_mma(low, ah, bl[j][0], bl[j][1], low);
 #pragma unroll
             for (int x = 0; x < 4; ++x) sum[j & 1][x] = j < 2 ? d[x] : sum[j & 1][x] + d[x];
           }
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             const float2 e2 = *(const float2*)&corr[16 * h2 + 8 * x + r][2 * c];
-            s[h][2 * x] = (fmaf(sum[0][2 * x] + sum[1][2 * x], inv2[0], bias2[0]) + e2.x) * a.scale;
-            s[h][2 * x + 1] =
-                (fmaf(sum[0][2 * x + 1] + sum[1][2 * x + 1], inv2[1], bias2[1]) + e2.y) * a.scale;
+            s[h][2 * x] = fmaf(sum[0][2 * x] + (sum[1][2 * x] + low[2 * x]), inv2[0], bias2[0]) + e2.x;
+            s[h][2 * x + 1] = fmaf(sum[0][2 * x + 1] + (sum[1][2 * x + 1] + low[2 * x + 1]), inv2[1], bias2[1]) + e2.y;
           }
         }
       }
@@ -562,16 +582,14 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
       asm volatile("cp.async.wait_group 1;" ::: "memory");  // the value half has landed
       __syncwarp();
 
-      // softmax over the strip; the largest norm sets the scale of the value operand
-      float nv[4][2], n_max = 0.0f;
+      // softmax over the strip, times the norms; a head's largest product sets the scale of its column of
+      // the value operand (the largest norm would not do: the probability in front of it may be
+      // any amount smaller, where a token of another strip dominates)
+      float nv[4][2], f[2], up_n[2], inv_n[2];
 #pragma unroll
       for (int h = 0; h < 4; ++h)
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          nv[h][x] = st.norms[16 * h + 8 * x + r];
-          n_max = fmaxf(n_max, nv[h][x]);
-        }
-      float f[2];
+        for (int x = 0; x < 2; ++x) nv[h][x] = st.norms[16 * h + 8 * x + r];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         float mx = -INFINITY;
@@ -581,15 +599,21 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
         for (int o = 4; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float m_new = fmaxf(m_run[x], mx);
         const bool any = m_new > -INFINITY;
-        f[x] = any ? __expf(m_run[x] - m_new) : 1.0f;
-        float sum = 0.0f;
+        f[x] = any ? tq_exp2(m_run[x] - m_new) : 1.0f;
+        float sum = 0.0f, most = 0.0f;
 #pragma unroll
         for (int h = 0; h < 4; ++h)
 #pragma unroll
           for (int y = 0; y < 2; ++y) {
-            s[h][2 * y + x] = any ? __expf(s[h][2 * y + x] - m_new) : 0.0f;
-            sum += s[h][2 * y + x];
+            const float e = any ? tq_exp2(s[h][2 * y + x] - m_new) : 0.0f;
+            sum += e;
+            s[h][2 * y + x] = e;
+            most = fmaxf(most, fabsf(e * nv[h][y]));
           }
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        up_n[x] = dp_lift(most, 13, inv_n[x]);
+        inv_n[x] *= inv_v;
         l_run[x] = l_run[x] * f[x] + sum;
         m_run[x] = m_new;
       }
@@ -598,20 +622,14 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
         acc[mt][0] *= f[0], acc[mt][1] *= f[1];
         acc[mt][2] *= f[0], acc[mt][3] *= f[1];
       }
-#pragma unroll
-      for (int o = 4; o <= 16; o <<= 1) n_max = fmaxf(n_max, __shfl_xor_sync(0xffffffffu, n_max, o));
-      float inv_n;
-      const float up_n = dp_lift(n_max, 13, inv_n);
-      inv_n *= inv_v;
 
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         uint32_t ph[2], pl[2];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {  // tokens 0-7, 8-15 of the tile
-          const float n = nv[h][x] * up_n;
           uint32_t hi, lo2;
-          dp_split(s[h][2 * x] * n, s[h][2 * x + 1] * n, hi, lo2);
+          dp_split_products(s[h][2 * x] * up_n[0], nv[h][x], s[h][2 * x + 1] * up_n[1], nv[h][x], hi, lo2);
           ph[x] = dp_transpose(hi);
           pl[x] = dp_transpose(lo2);
         }
@@ -652,7 +670,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
           float d[4];
           dp_product(d, ah, al, ph, pl);
 #pragma unroll
-          for (int x = 0; x < 4; ++x) acc[mt][x] = fmaf(d[x], inv_n, acc[mt][x]);
+          for (int x = 0; x < 4; ++x) acc[mt][x] = fmaf(d[x], inv_n[x & 1], acc[mt][x]);
         }
       }
       __syncwarp();  // the value half has been read
@@ -703,7 +721,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
     };
     group_sync();  // (what the group did before in this memory is over)
     copy_rows(a.hot_k, t_lo, min(DP_HOT, t_hi - t_lo));
-    load_q(unit, gt);
+    load_q(unit, gt, false);  // (products of 16-bit numbers are exact: the sum is scaled)
     float m_h[2], l_h[2];  // of heads 2 warp + i, the same in every lane
     unsigned long long av[NP];  // channel gtid
 #pragma unroll
@@ -762,8 +780,8 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             const float2 e = dp_unpack(dp_add2(low[x], dot[x]));
-            ht.s[h4 + 2 * x][tok] = e.x * a.scale;
-            ht.s[h4 + 2 * x + 1][tok] = e.y * a.scale;
+            ht.s[h4 + 2 * x][tok] = tq_scaled<true>(e.x);
+            ht.s[h4 + 2 * x + 1][tok] = tq_scaled<true>(e.y);
           }
         }
       }
@@ -782,11 +800,11 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
         for (int o = 16; o >= 1; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float m_new = fmaxf(m_h[i], mx);
         const bool any = m_new > -INFINITY;
-        const float fo = any ? __expf(m_h[i] - m_new) : 1.0f;
+        const float fo = any ? tq_exp2(m_h[i] - m_new) : 1.0f;
         float sum = 0.0f;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-          const float pv = any && lane + 32 * x < n_tok ? __expf(sc[x] - m_new) : 0.0f;
+          const float pv = any && lane + 32 * x < n_tok ? tq_exp2(sc[x] - m_new) : 0.0f;
           sum += pv;
           ht.p[lane + 32 * x][gg] = pv;
         }
