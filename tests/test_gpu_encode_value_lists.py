@@ -64,3 +64,37 @@ def test_a_tile_that_is_not_encoded_is_stored_as_zeros(dt, vb):
     ctx.clear(0, 0)
     ctx.append(0, x, x)
     assert ctx.status() == 0 and torch.equal(ctx.dequant(0, 0, 0, n)[1], want)
+
+
+@pytest.mark.parametrize("dt", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("vb", [3, 4])
+def test_sums_that_cancel_near_a_boundary(dt, vb):
+    """Rows that put one channel on a boundary by two large parts of opposite sign: where the tensor cores'
+    sums are least exact and a wrong code is nearest."""
+    import numpy as np
+    import torch
+
+    from turboquant_pro_b200 import KVContext
+    from turboquant_pro_b200.context import value_codebook
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(11)
+    h, n = 4, 4096
+    pi = torch.from_numpy(np.asarray(KVContext(
+        n_layers=1, n_seqs=1, n_kv_heads=1, n_q_heads=1, value_bits=vb, hot_window=512,
+        max_tokens_per_seq=600, kv_dtype=dt, seed=3).pi, dtype=np.float32)).cuda().double()
+    bounds = torch.from_numpy(np.asarray(value_codebook(128, vb)[1])).cuda().double()
+    row = pi[torch.randint(0, 128, (n, h), device="cuda", generator=gen)]
+    first = torch.arange(128, device="cuda") < 64
+    n1 = (row * row * first).sum(-1)
+    n2 = (row * row * ~first).sum(-1)
+    b = bounds[torch.randint(0, len(bounds), (n, h), device="cuda", generator=gen)]
+    # (n1 - s n2) / sqrt(n1 + s^2 n2) = b, for s of the sign that cancels
+    lo, hi = torch.full_like(n1, -50.0), torch.full_like(n1, 50.0)
+    for _ in range(60):
+        mid = (lo + hi) / 2
+        above = (n1 - mid * n2) / (n1 + mid * mid * n2).sqrt() > b
+        lo, hi = torch.where(above, mid, lo), torch.where(above, hi, mid)
+    v = torch.where(first, row, -lo[..., None] * row).to(getattr(torch, dt))[None]
+    a, b = _values(v, (n,), h, vb, 512, dt)
+    assert a == b
