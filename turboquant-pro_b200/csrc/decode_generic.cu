@@ -614,7 +614,12 @@ int tq_launch_decode(tq_ctx* ctx, int layer, const void* q, int q_dtype, int blo
     const long share = std::max((total_nb * g.n_kv_heads * ((g.group + 7) / 8) + groups - 1) / groups, 1l);
     ns_cold = max_nb > 0 ? (int)std::min<long>(std::max((max_nb - 1) / share + 3, 2l), g.max_splits - ns_hot) : 0;
   }
-  if (ns_cold + ns_hot == 0) ns_hot = 1;  // empty layer: the kernels still write zeros
+  // A captured launch may be replayed on longer sequences: the kernels go by the lengths on the device, so
+  // there is room for partials of pages and of the window wherever the call asks for any.
+  if (with_hot) ns_hot = std::max(ns_hot, 1);
+  if (ns_cold == 0 && g.max_blocks > 0 && (block_end < 0 || block_end > block_begin))
+    ns_cold = tq_decode_pages_form(g) ? 2 : 1;
+  if (ns_cold + ns_hot == 0) ns_hot = 1;  // nothing asked for: the kernels still write zeros
   a.ns_cold = ns_cold;
   a.ns_hot = ns_hot;
 
@@ -724,7 +729,8 @@ extern "C" int32_t tq_decode_static_scratch(tq_ctx* ctx, int32_t layer, const vo
   int ns_hot = max_hot > 0 ? std::min((max_hot + 127) / 128, 2) : 0;
   int ns_cold = max_nb > 0 ? std::min(max_nb, TQ_STATIC_SLOTS - ns_hot) : 0;
   if (tq_decode_pages_form(g) && ns_cold > 0) ns_cold = TQ_STATIC_SLOTS - ns_hot;
-  if (ns_cold + ns_hot == 0) ns_hot = 1;  // empty layer: the kernels still write zeros
+  ns_hot = std::max(ns_hot, 1);
+  if (ns_cold == 0 && g.max_blocks > 0) ns_cold = tq_decode_pages_form(g) ? 2 : 1;  // (as in tq_launch_decode)
   a.ns_cold = ns_cold;
   a.ns_hot = ns_hot;
 
