@@ -54,3 +54,19 @@ def test_forms_and_damage():
     assert kv_blob._read_native(_lib.load(), many, 1 << 20, True) is None  # (left to numpy)
     with np.load(io.BytesIO(many)) as z:
         assert len(z.files) == 70
+
+
+def test_prototypes_of_other_packages_are_left_alone():
+    """ctypes.pythonapi is shared by the whole process: its attributes are neither changed nor relied on."""
+    import ctypes
+
+    shared = ctypes.pythonapi.PyBytes_FromStringAndSize
+    before = shared.restype, shared.argtypes
+    assert before != (ctypes.py_object, [ctypes.c_void_p, ctypes.c_ssize_t])
+    arrays = {"a": np.arange(1000, dtype=np.int32)}
+    want = kv_blob._write_npz(arrays)
+    try:
+        shared.restype, shared.argtypes = ctypes.c_int, [ctypes.c_char_p, ctypes.c_int]
+        assert kv_blob._write_npz(arrays) == want
+    finally:
+        shared.restype, shared.argtypes = before

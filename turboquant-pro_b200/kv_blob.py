@@ -152,8 +152,9 @@ def _native():
         return None
 
 
-_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.restype, _new_bytes.argtypes = ctypes.py_object, [ctypes.c_void_p, ctypes.c_ssize_t]
+# (a function object of its own: the attributes of ctypes.pythonapi belong to the whole process)
+_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
 
 
 def _address(a) -> int:
