@@ -425,7 +425,7 @@ int32_t tq_debug_wait(tq_ctx* ctx, int32_t wait_limit, int32_t withhold_tile);
 /* How near to a boundary of the codebook a product of the value encoder for 128- and 256-token blocks may
  * lie before its code is computed a second time, in the reference's order of operations (core.py:246-260
  * has the rotation; no counterpart).  For the test of the bound. */
-float tq_debug_value_slack(int32_t kv_dtype);
+float tq_debug_value_slack(void);
 
 /* Pipeline trace of the tensor-core decode kernel (debugging aid, no counterpart in the
  * reference).  `on` switches stamping on or off for later tq_decode calls; if `stamps` is

@@ -125,7 +125,7 @@ SIGNATURES = {
     "tq_set_key_mean_mask": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "tq_set_key_bias_means": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "tq_debug_trace": (C.c_int32, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]),
-    "tq_debug_value_slack": (C.c_float, [C.c_int32]),
+    "tq_debug_value_slack": (C.c_float, []),
     "tq_profile_enable": (C.c_int32, [C.c_void_p, C.c_int32]),
     "tq_npz_write": (C.c_int64, [C.c_int32, C.c_void_p, C.c_char_p, C.c_void_p, C.c_int64]),
     "tq_npz_read": (C.c_int32, [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p]),

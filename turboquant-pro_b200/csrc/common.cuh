@@ -111,7 +111,7 @@ struct ValueTable {
   uint32_t slack, zero_code;
   float scale;
 };
-void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable* vt);
+void tq_value_table(const float* boundaries, int bits, ValueTable* vt);
 
 struct tq_ctx {
   tq_geom g;

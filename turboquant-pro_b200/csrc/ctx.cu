@@ -203,7 +203,7 @@ int32_t tq_ctx_create(const tq_geom* g, const tq_buffers* bufs, int32_t device, 
   c->last_launches = 0;
   std::memcpy(c->h_centroids, t->centroids, sizeof(c->h_centroids));
   std::memcpy(c->h_boundaries, t->boundaries, sizeof(c->h_boundaries));
-  tq_value_table(c->h_boundaries, g->value_bits, g->kv_dtype, &c->value_table);
+  tq_value_table(c->h_boundaries, g->value_bits, &c->value_table);
   delete t;
   *out = c;
   return TQ_OK;

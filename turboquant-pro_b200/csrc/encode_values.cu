@@ -26,7 +26,7 @@
 // distance to the boundary in the bits under it: one funnel shift appends the code, one compare
 // finds the distances within the slack.
 //
-// Those products (see value_slack) go on a list of the warp's own: (row, destination, norm, channel,
+// Those products (see VALUE_SLACK) go on a list of the warp's own: (row, destination, norm, channel,
 // token, code).  Four more warps take them from there, compute them again in the reference's order, a
 // lane per entry, and flip the bits of a code that differs in the page.  (The epilogue warps must not
 // do it themselves: a batch takes as long as several tiles, and the other warps would wait at the
@@ -46,15 +46,16 @@ namespace {
 // The exact dot product lies within 127 * 2^-25 + 2^-23 < 4.0e-6 of the reference's sum (the running
 // sum stays below 1: the absolute values of the terms add up to at most |u| |row of Pi| = 1).
 // Here Pi is two fp16 parts (what is left is below 2^-23 of a term; of float32 rows likewise) or, for
-// bfloat16 rows, two bfloat16 parts (2^-18 of a term, 3.9e-6 in all).  The products with a low part come
-// first; their sums stay below 2^-9 and lose next to nothing.  Then the accumulator takes eight steps of
+// bfloat16 rows, three bfloat16 parts (2^-26).  The products with a low part come
+// first; their sums stay below 2^-8 and lose next to nothing.  Then the accumulator takes eight steps of
 // 16 terms; a step that aligns its 17 addends to the largest of them and cuts them off 24 bits below
-// loses at most 17 * 2^-24, 8.2e-6 in all.  Together 1.24e-5, for bfloat16 1.62e-5.
+// loses at most 17 * 2^-24, 8.2e-6 in all.  Together 1.24e-5.
 // How the tensor cores align and cut is not documented, so the slack is two and a half times that, as in
 // the other encoders.  (Measured, on 1.1e9 products whose partial sums are large and cancel: a slack of
-// zero gives other codes up to 2.2e-7 from a boundary with fp16 parts and 7.3e-7 with bfloat16 ones.)  8 x
-// 16 384 fp16 tokens x 8 heads, 3 bits: a prompt takes 547 us with this slack, 521 with 1.13 times the bound.
-TQ_HD float value_slack(int dt) { return dt == TQ_BF16 ? 4.1e-5f : 3.1e-5f; }
+// zero gives other codes up to 2.2e-7 from a boundary, 7.3e-7 where Pi had two bfloat16 parts.)  Microseconds of an
+// append of 8 x 16 384 tokens x 8 heads: fp16, 3 bits, 451 with 1.13 times the bound and 477 with this;
+// bfloat16, 4 bits, 617 with two parts of Pi and two and a half times their bound, 563 with three parts.
+constexpr float VALUE_SLACK = 3.1e-5f;
 
 constexpr int EV_LOADERS = 256;              // threads of the loader warps
 constexpr int EV_EPI_WARPS = 12;
@@ -62,7 +63,7 @@ constexpr int EV_REDO_WARPS = 4;
 constexpr int EV_THREADS = EV_LOADERS + 32 * (EV_EPI_WARPS + EV_REDO_WARPS);
 constexpr int EV_PER_REDO = EV_EPI_WARPS / EV_REDO_WARPS;  // lists a redo warp takes from
 constexpr int EV_LIST = 64;                  // entries of a list (a ring)
-constexpr int EV_PI_BYTES = 2 * TQ_D * TQ_D * 2;
+constexpr int EV_PI_PART = TQ_D * TQ_D * 2;  // bytes of one part of Pi
 constexpr int EV_TILE_BYTES = 33280;         // rows of a tile: 128 x 256 or 64 x 512 bytes, and the pads
 constexpr int EV_WAIT = 1 << 20;             // probes of a barrier (2 us each at most) before a wait gives up
 constexpr int EV_WITHHOLD = 1 << 20;         // test hook: a.withhold_row of tile 0 of the first CTA
@@ -72,9 +73,13 @@ struct EvShape {
   static constexpr bool F32 = DT == TQ_F32;
   static constexpr int T = F32 ? 64 : 128;      // tokens of a tile
   static constexpr int PS = 16 * T + 16;        // bytes from one piece of the rows to the next (padded)
-  static constexpr int SLOTS = F32 ? 2 : 4;     // tiles between loader and epilogue
-  static constexpr int RAW = F32 ? 2 : 4;       // row buffers (16-bit: they are the operands)
-  static constexpr int COLS = F32 ? 128 : 512;  // columns of tensor memory: SLOTS * T
+  // Parts of Pi: two of fp16 or three of bfloat16 hold 22 and 24 bits.  (Where there are three, shared memory
+  // has room for three tiles.)
+  static constexpr int PARTS = DT == TQ_BF16 ? 3 : 2;
+  static constexpr int SLOTS = F32 ? 2 : PARTS == 3 ? 3 : 4;  // tiles between loader and epilogue
+  static constexpr int RAW = SLOTS;             // row buffers (16-bit: they are the operands)
+  static constexpr int TILES = F32 ? 4 : SLOTS; // tile buffers
+  static constexpr int COLS = F32 ? 128 : 512;  // columns of tensor memory: SLOTS * T, a power of two
 };
 
 struct EvInfo {            // what the epilogue needs to know about a tile
@@ -92,9 +97,10 @@ struct EvList {
   uint32_t meta[EV_LIST];  // channel | token << 8 | code << 12
 };
 
+template <int DT>
 struct EvShared {
-  alignas(16) uint8_t pi[EV_PI_BYTES];  // Pi as A operand: [hi | lo][K / 8][128 rows][8]
-  alignas(16) uint8_t tile[4][EV_TILE_BYTES];  // rows; float32: two row buffers, two operand buffers
+  alignas(16) uint8_t pi[EvShape<DT>::PARTS * EV_PI_PART];  // Pi as A operand: [hi | lo ...][K / 8][128 rows][8]
+  alignas(16) uint8_t tile[EvShape<DT>::TILES][EV_TILE_BYTES];  // rows; float32: two row buffers, two operand buffers
   // per slot and token: z = product * mul + 1/2; -1: no usable norm; -2: a row of zeros
   alignas(16) float mul[4][128];
   float norm[4][128];
@@ -106,7 +112,9 @@ struct EvShared {
   uint32_t tmem;
   int lost;  // first tile whose codes or norms are not all there: a wait ran out
 };
-static_assert(sizeof(EvShared) <= 227 * 1024, "shared memory of one CTA");
+static_assert(sizeof(EvShared<TQ_F32>) <= 227 * 1024 && sizeof(EvShared<TQ_F16>) <= 227 * 1024 &&
+                  sizeof(EvShared<TQ_BF16>) <= 227 * 1024,
+              "shared memory of one CTA");
 
 TQ_DEV void ev_cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -176,7 +184,8 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   constexpr int VGB = TQ_GROUP_TOK * TQ_D * VB / 8;
   const tq_geom& g = a.g;
   extern __shared__ __align__(128) uint8_t ev_smem[];
-  EvShared& sh = *(EvShared*)ev_smem;
+  using Shared = EvShared<DT>;
+  Shared& sh = *(Shared*)ev_smem;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* pi_rows = a.tables->pi;
   const bool keys = a.polar_keys_pass != 0;
@@ -205,7 +214,12 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
       ev_split<DT>(make_float2(p[k].x * ev_pi_scale<DT>(), p[k].y * ev_pi_scale<DT>()), hi, lo);
       uint32_t* at = (uint32_t*)(sh.pi + (d >> 3) * 2048 + m * 16 + (d & 7) * 2);
       at[0] = hi;
-      at[EV_PI_BYTES / 8] = lo;
+      at[EV_PI_PART / 4] = lo;
+      if constexpr (Sh::PARTS == 3) {
+        const float2 h = ev_pair<DT>(hi), l = ev_pair<DT>(lo);
+        const __nv_bfloat162 r = __floats2bfloat162_rn(p[k].x - h.x - l.x, p[k].y - h.y - l.y);
+        at[EV_PI_PART / 2] = *(const uint32_t*)&r;
+      }
     }
   }
   if (threadIdx.x < SLOTS) {
@@ -352,13 +366,19 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + (uint32_t)((i % SLOTS) * T);
       const uint64_t a_hi0 = umma_desc_k_major(enc_smem(sh.pi), 2048, 128);
-      const uint64_t a_lo0 = umma_desc_k_major(enc_smem(sh.pi) + EV_PI_BYTES / 2, 2048, 128);
+      const uint64_t a_lo0 = umma_desc_k_major(enc_smem(sh.pi) + EV_PI_PART, 2048, 128);
       const uint64_t b0 = umma_desc_k_major(
-          enc_smem(sh.tile[F32 ? 2 + i % 2 : i % 4]), PS, 128);
+          enc_smem(sh.tile[F32 ? 2 + i % 2 : i % Sh::TILES]), PS, 128);
       constexpr uint64_t KA = 4096 >> 4, KB = 2 * PS >> 4;  // a step of 16 input channels
+      // the small products first (see VALUE_SLACK)
+      if constexpr (Sh::PARTS == 3) {
+        const uint64_t a_rest0 = umma_desc_k_major(enc_smem(sh.pi) + 2 * EV_PI_PART, 2048, 128);
 #pragma unroll
-      for (int kb = 0; kb < 8; ++kb) {  // the small products first (see value_slack)
-        ev_mma(d, a_lo0 + kb * KA, b0 + kb * KB, idesc, kb > 0);
+        for (int kb = 0; kb < 8; ++kb) ev_mma(d, a_rest0 + kb * KA, b0 + kb * KB, idesc, kb > 0);
+      }
+#pragma unroll
+      for (int kb = 0; kb < 8; ++kb) {
+        ev_mma(d, a_lo0 + kb * KA, b0 + kb * KB, idesc, kb > 0 || Sh::PARTS == 3);
         if (F32) ev_mma(d, a_hi0 + kb * KA, b0 + kb * KB + (EV_TILE_BYTES / 2 >> 4), idesc, 1u);
       }
 #pragma unroll
@@ -376,10 +396,16 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     for (int i = 0; i < n; ++i) {
       const int slot = i % SLOTS;
       if (!F32) {
-        if (more && fetch(n)) ++n;
-        else more = false;
-        commit();
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        // With three slots the next copies start behind this tile's products: they wait for the epilogue of
+        // the tile before it.
+        if (SLOTS > 3) {
+          if (more && fetch(n)) ++n;
+          else more = false;
+          commit();
+          asm volatile("cp.async.wait_group 2;" ::: "memory");
+        } else {
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         sync();
         if (tl == 0) issue(i);
@@ -428,6 +454,13 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
         }
         const bool all_sane = __all_sync(0xffffffffu, sane);
         if (lane == 0) ((uint8_t*)&sh.odd[slot])[warp] = all_sane ? 0 : 1;
+        if (SLOTS == 3) {
+          mbar_arrive(enc_smem(&sh.full[slot]));
+          if (more && fetch(n)) ++n;
+          else more = false;
+          commit();
+          continue;
+        }
       } else {
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         sync();
@@ -794,7 +827,7 @@ int launch_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys, int
   static bool attr_set[16] = {};  // per device: the attribute belongs to the device's context
   if (!attr_set[device & 15]) {
     TQ_CUDA(cudaFuncSetAttribute(encode_values_tile_kernel<DT, VB>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EvShared)));
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EvShared<DT>)));
     attr_set[device & 15] = true;
   }
   const long total = (long)a.seq_count * a.g.n_kv_heads * a.max_new_blocks *
@@ -809,7 +842,7 @@ int launch_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys, int
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)std::min<long>(total, sm_count));
   cfg.blockDim = dim3(EV_THREADS);
-  cfg.dynamicSmemBytes = sizeof(EvShared);
+  cfg.dynamicSmemBytes = sizeof(EvShared<DT>);
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = after_keys ? 1 : 0;
@@ -819,7 +852,7 @@ int launch_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys, int
 
 }  // namespace
 
-void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable* vt) {
+void tq_value_table(const float* boundaries, int bits, ValueTable* vt) {
   // the widest range of y that holds all boundaries and whose 32 bins hold at most one each, with the slack
   // on both sides
   const int n = (1 << bits) - 1;
@@ -828,7 +861,7 @@ void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable*
     if (!(std::fabs(boundaries[i]) < 1.0f) || (i > 0 && !(boundaries[i] > boundaries[i - 1]))) return;
   for (double range = 1.0; range > 0.02 && !vt->ok; range *= 0.99) {
     const double unit = VALUE_SPAN * 8388608.0 / (2.0 * range);  // Z per y
-    const long slack = (long)std::ceil(value_slack(kv_dtype) * unit) + 2;
+    const long slack = (long)std::ceil(VALUE_SLACK * unit) + 2;
     long at[15];
     int touched = 0;  // last bin the boundaries so far can lie in; the first and the last bin have none
     bool fits = slack < (1 << 17);
@@ -859,7 +892,7 @@ void tq_value_table(const float* boundaries, int bits, int kv_dtype, ValueTable*
   }
 }
 
-extern "C" float tq_debug_value_slack(int32_t kv_dtype) { return value_slack(kv_dtype); }
+extern "C" float tq_debug_value_slack() { return VALUE_SLACK; }
 
 int tq_launch_encode_values_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys,
                                   int sm_count, int device, cudaStream_t st) {
