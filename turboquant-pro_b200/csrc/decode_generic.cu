@@ -11,6 +11,11 @@
 
 namespace {
 
+// whether a sequence of the context can ever have a compressed block
+bool may_have_pages(const tq_geom& g) {
+  return n_cold_blocks(g.max_tokens_per_seq, g.hot_window, g.block_tokens) > 0;
+}
+
 TQ_DEV float ld_any(const void* p, size_t i, int dt) {
   if (dt == TQ_F32) return ((const float*)p)[i];
   if (dt == TQ_F16) return __half2float(((const __half*)p)[i]);
@@ -617,7 +622,7 @@ int tq_launch_decode(tq_ctx* ctx, int layer, const void* q, int q_dtype, int blo
   // A captured launch may be replayed on longer sequences: the kernels go by the lengths on the device, so
   // there is room for partials of pages and of the window wherever the call asks for any.
   if (with_hot) ns_hot = std::max(ns_hot, 1);
-  if (ns_cold == 0 && g.max_blocks > 0 && (block_end < 0 || block_end > block_begin))
+  if (ns_cold == 0 && may_have_pages(g) && (block_end < 0 || block_end > block_begin))
     ns_cold = tq_decode_pages_form(g) ? 2 : 1;
   if (ns_cold + ns_hot == 0) ns_hot = 1;  // nothing asked for: the kernels still write zeros
   a.ns_cold = ns_cold;
@@ -730,7 +735,7 @@ extern "C" int32_t tq_decode_static_scratch(tq_ctx* ctx, int32_t layer, const vo
   int ns_cold = max_nb > 0 ? std::min(max_nb, TQ_STATIC_SLOTS - ns_hot) : 0;
   if (tq_decode_pages_form(g) && ns_cold > 0) ns_cold = TQ_STATIC_SLOTS - ns_hot;
   ns_hot = std::max(ns_hot, 1);
-  if (ns_cold == 0 && g.max_blocks > 0) ns_cold = tq_decode_pages_form(g) ? 2 : 1;  // (as in tq_launch_decode)
+  if (ns_cold == 0 && may_have_pages(g)) ns_cold = tq_decode_pages_form(g) ? 2 : 1;  // (as in tq_launch_decode)
   a.ns_cold = ns_cold;
   a.ns_hot = ns_hot;
 
