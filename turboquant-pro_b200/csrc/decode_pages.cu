@@ -882,11 +882,11 @@ int launch_pages(const DecodeArgs& a, int ctas, cudaStream_t st) {
 // Tiles of eight heads; a group of five to seven leaves up to three idle, one of nine to fifteen up to
 // seven of its second tile.  Microseconds of a decode call, general kernel / this one, merge included
 // (K4/V3, bf16; 64 units of 700 to 12 000 tokens, 64 of 6 000, 8 of 32 768, 32 of 900, 4 of 600):
-//   5 heads   258 / 78   269 / 68   199 / 55   44 / 23   40 / 21
-//   7 heads   260 / 80   271 / 71   200 / 54   44 / 23   40 / 21
-//   9 heads   558 / 126  562 / 114  390 / 77   75 / 32   65 / 21
-//  16 heads   557 / 134  560 / 113  387 / 81   79 / 33   66 / 21
-// What bounds it: the look-ups (shared memory) and the issue slots of the splits and products.
+//   5 heads   258 / 80   269 / 72   199 / 54   44 / 23   40 / 21
+//   7 heads   260 / 80   271 / 72   200 / 54   44 / 24   40 / 22
+//   9 heads   558 / 128  562 / 119  390 / 80   75 / 34   65 / 23
+//  16 heads   557 / 137  560 / 121  387 / 81   79 / 35   66 / 23
+// What bounds it: the look-ups (shared memory 56 %) and the issue slots (50 %) of splits and products.
 int tq_launch_decode_pages(const DecodeArgs& a, int sm_count, cudaStream_t st) {
   return a.g.value_bits == 3 ? launch_pages<3>(a, sm_count, st) : launch_pages<4>(a, sm_count, st);
 }

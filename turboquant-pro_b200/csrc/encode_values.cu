@@ -5,7 +5,14 @@
 //   y_ch = sequential, unfused sum over d of fl(x_d / max(norm, 1e-30)) * Pi[ch][d]
 //   code = #{ j : boundary_j < y_ch }
 //
-// One persistent CTA per SM, warps by role; they meet through mbarriers only (all waits bounded):
+// One persistent CTA per SM, warps by role.  The roles meet through mbarriers and the counts of the lists, and
+// those waits are bounded.  Three others are not: the loaders' named barrier (its eight warps run the same
+// loop, whose length follows from the sequence lengths alone), the block barrier at the end (every role
+// gets there: its loops are over tiles or bounded waits), and the allocation of tensor memory, which
+// waits for other CTAs of this kernel or of encode_values_tc5_kernel on the SM; those free it without
+// waiting for any other kernel, and shared memory has room for one of them at a time anyway.
+// Warp-wide operations stand only where all lanes decided alike (votes, or one lane's reading).
+//
 //
 // * Eight loader warps copy a tile of 128 tokens (64 for float32) into shared memory with cp.async,
 //   two tiles ahead, straight into the tensor cores' operand layout, [16-byte piece][token], which two
@@ -32,9 +39,11 @@
 // do it themselves: a batch takes as long as several tiles, and the other warps would wait at the
 // ring of slots.)
 //
-// What bounds it (8 x 16 384 tokens x 8 heads, 3 bits, 224 us): the logic pipe and the chains of the epilogue
-// (switched off: 165 us without lists and their recomputation, 124 without codes, products and norms, 83
-// without the copies, too); 42 % of the issue slots, six warps a scheduler.
+// What bounds it (8 x 16 384 tokens x 8 heads): at 3 bits (246 us) the logic pipe and the chains of the
+// epilogue, 49 % of the issue slots, six warps a scheduler; at 4 bits (328 us in bfloat16) the warps that
+// recompute, which wait for rows in global memory and divide.  (With a slack of 1.4e-5, 3 bits, 224 us; of
+// that 165 without lists and their recomputation, 124 without codes, products and norms, too, 83 without the
+// copies.)
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -819,8 +828,9 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
 }
 
 // Microseconds of the value encoder, groups of 16 tokens (encode_values_tc5_kernel) / this one: 8 x 16 384 fp16
-// tokens x 8 heads, 3 bits, 566 / 224; bf16, 4 bits, 612 / 247; 4 001 float32 tokens x 32 heads, 4 bits, 92 / 62;
-// 3 333 bf16 tokens x 8 heads, 4 bits, 33 / 24; 4 x 1 010, 3 bits, 32 / 20.
+// tokens x 8 heads, 3 bits, 561 / 246; bf16, 4 bits, 616 / 328, 3 bits 563 / 250.  Of a whole append, where this
+// one starts under the key encoder: 814 / 477, 870 / 563, 819 / 485; 4 001 float32 tokens x 32 heads, 4 bits,
+// 164 / 131; 3 333 bf16 tokens x 8 heads, 4 bits, 58 / 46; 4 x 1 010, 3 bits, 58 / 46; one block of 8 heads 48 / 31.
 template <int DT, int VB>
 int launch_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys, int sm_count, int device,
                  cudaStream_t st) {
@@ -834,8 +844,8 @@ int launch_tiles(const EncodeArgs& a, const ValueTable& vt, bool after_keys, int
                      (a.g.block_tokens / EvShape<DT>::T);
   // It may start while the key encoder before it in the stream drains (they share no output); it ends
   // after that kernel has, so that the ring writer, which waits for this one, follows both.
-  // An append of 3 333 bf16 tokens x 8 heads 53 -> 47 us, 4 001 float32 tokens x 32 heads 138 -> 132, 8 x 16 384
-  // fp16 tokens 484 -> 475.
+  // (An append of 3 333 bf16 tokens x 8 heads 53 -> 47 us, 4 001 float32 tokens x 32 heads 138 -> 132, 8 x 16 384
+  // fp16 tokens 484 -> 475, with the slack that was smaller then.)
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
