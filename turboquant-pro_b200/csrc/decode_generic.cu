@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(TQ_D) combine_kernel(DecodeArgs a) {
   __syncthreads();
   float L = 0.0f, C = 0.0f, Hh = 0.0f;
   auto add = [&](int s, float y) {
-    const float v = s_m[s] > -INFINITY ? y * s_w[s] : 0.0f;  // (an empty partial has no sums)
+    const float v = s_l[s] < 0.0f ? 0.0f : y * s_w[s];  // (marked: no sums.  Others count, a NaN among them)
     L += s_l[s] * s_w[s];
     if (s < a.ns_cold)
       C += v;

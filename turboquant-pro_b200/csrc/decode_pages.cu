@@ -282,12 +282,12 @@ __global__ void __launch_bounds__(DP_THREADS, 1) decode_pages_kernel(DecodeArgs 
   auto slot_of = [&](int unit, int gt, int slot) -> float* {
     return a.partials + (((size_t)unit * g.max_splits + slot) * G + gt * GT) * TQ_PART_STRIDE;
   };
-  auto mark_empty = [&](int unit, int gt, int first, int end) {  // partials that hold nothing
+  auto mark_empty = [&](int unit, int gt, int first, int end) {  // partials without sums (a sum below zero says so)
     for (int i = gtid; i < (end - first) * GT; i += DP_GTH)
       if (gt * GT + i % GT < G) {
         float* pp = slot_of(unit, gt, first + i / GT) + (i % GT) * TQ_PART_STRIDE;
         pp[0] = -INFINITY;
-        pp[1] = 0.0f;
+        pp[1] = -1.0f;
       }
   };
   if (a.ns_cold > 0)
